@@ -654,8 +654,11 @@ static int launch_variant(const UpdArgs &a, cudaStream_t s, bool met, int varian
   if (variant == U1V_QUAD) {
     threads = std::min(threads, 128);  // the kernel's launch bound
     const int blocks = u1i::blocks_for(a.g.Vh / 4, threads);
-    return met ? launch_pdl(k_update_quad<D, MU, true, SRC>, blocks, s, a, "k_update_quad", threads)
-               : launch_pdl(k_update_quad<D, MU, false, SRC_PHILOX>, blocks, s, a, "k_update_quad", threads);
+    if (a.ctas == 7)
+      return met ? launch_pdl(k_update_quad<D, MU, true, SRC, 7>, blocks, s, a, "k_update_quad", threads)
+                 : launch_pdl(k_update_quad<D, MU, false, SRC_PHILOX, 7>, blocks, s, a, "k_update_quad", threads);
+    return met ? launch_pdl(k_update_quad<D, MU, true, SRC, 6>, blocks, s, a, "k_update_quad", threads)
+               : launch_pdl(k_update_quad<D, MU, false, SRC_PHILOX, 6>, blocks, s, a, "k_update_quad", threads);
   }
   if (variant == U1V_PAIR32 || variant == U1V_PAIR) {
     const int blocks = u1i::blocks_for(a.g.Vh / 2, threads);
@@ -693,18 +696,23 @@ static int launch_phase(const UpdArgs &a, cudaStream_t s, bool met, int src, int
   return fail(U1_ERR_INVALID, "k_update: direction out of range");
 }
 
-// Whether a four-site phase at the lattice's block size runs as a single
-// wave (the SM-local block order then applies); cached per block size.
+// How four-site phases at the lattice's block size run: 6 blocks of 128
+// threads per SM, or 7 where that makes the phase a single wave; a single
+// wave takes its blocks in the SM-local order.  Cached per block size.
 static void quad_layout(u1_lattice *lat) {
   if (lat->remap_block == lat->block) return;
   const int sms = lat->ctx->prop.multiProcessorCount;
   const int threads = std::min(lat->block, 128);
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_update_quad<4, 0, false, SRC_PHILOX>, threads, 0) !=
-      cudaSuccess)
-    per_sm = 0;
+  int per6 = 0, per7 = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per6, k_update_quad<4, 0, false, SRC_PHILOX, 6>, threads, 0) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per7, k_update_quad<4, 0, false, SRC_PHILOX, 7>, threads, 0) !=
+          cudaSuccess)
+    per6 = per7 = 0;
   const long long blocks = ((long long)lat->g.Vh / 4 + threads - 1) / threads;
-  lat->remap_sms = (per_sm > 0 && blocks <= (long long)per_sm * sms) ? sms : 0;
+  const bool wave6 = blocks <= (long long)per6 * sms, wave7 = blocks <= (long long)per7 * sms;
+  lat->quad_ctas = (wave7 && !wave6) ? 7 : 6;
+  lat->remap_sms = (wave6 || wave7) ? sms : 0;
   lat->remap_block = lat->block;
 }
 
@@ -734,6 +742,15 @@ static int sm_remap(u1_lattice *lat) {
   }();
   quad_layout(lat);
   return off ? 0 : lat->remap_sms;
+}
+
+// The four-site kernels' blocks per SM and block order into the kernel
+// arguments (launch order when `plain`); returns the SM count of the order.
+static int set_quad(UpdArgs &a, u1_lattice *lat, bool plain) {
+  const int sms = plain ? (quad_layout(lat), 0) : sm_remap(lat);
+  a.ctas = lat->quad_ctas;
+  a.order = sm_order(u1i::blocks_for(lat->g.Vh / 4, std::min(lat->block, 128)), sms);
+  return sms;
 }
 
 // The proposal settings of `lat` into the kernel arguments.
@@ -865,10 +882,18 @@ static int launch_meas_phase_mu(const UpdArgs &a, cudaStream_t s, bool met, bool
   cfg.numAttrs = 1;
   double *slot = partials + (size_t)(MU - 1) * meas_phase_blocks(a.g) * 2;
   cudaError_t e;
-  if (quad)
-    e = !met ? cudaLaunchKernelEx(&cfg, k_update_quad_meas<D, MU, false>, a, slot)
-        : win ? cudaLaunchKernelEx(&cfg, k_update_quad_meas<D, MU, true, SRC_WINDOW>, a, slot)
-              : cudaLaunchKernelEx(&cfg, k_update_quad_meas<D, MU, true>, a, slot);
+  if (quad) {
+    UpdArgs q = a;
+    q.order = sm_order((int)cfg.gridDim.x, a.order.S);  // these blocks hold 128 threads whatever the lattice's block size
+    if (a.ctas == 7)
+      e = !met ? cudaLaunchKernelEx(&cfg, k_update_quad_meas<D, MU, false, SRC_PHILOX, 7>, q, slot)
+          : win ? cudaLaunchKernelEx(&cfg, k_update_quad_meas<D, MU, true, SRC_WINDOW, 7>, q, slot)
+                : cudaLaunchKernelEx(&cfg, k_update_quad_meas<D, MU, true, SRC_PHILOX, 7>, q, slot);
+    else
+      e = !met ? cudaLaunchKernelEx(&cfg, k_update_quad_meas<D, MU, false, SRC_PHILOX, 6>, q, slot)
+          : win ? cudaLaunchKernelEx(&cfg, k_update_quad_meas<D, MU, true, SRC_WINDOW, 6>, q, slot)
+                : cudaLaunchKernelEx(&cfg, k_update_quad_meas<D, MU, true, SRC_PHILOX, 6>, q, slot);
+  }
   else if ((a.g.hN0 & 1) == 0)
     e = !met ? cudaLaunchKernelEx(&cfg, k_update_pair_meas<D, MU, false>, a, slot)
         : win ? cudaLaunchKernelEx(&cfg, k_update_pair_meas<D, MU, true, SRC_WINDOW>, a, slot)
@@ -964,8 +989,8 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
 #endif
   // with a freeze period the SM-local order would hand whole frozen slabs to
   // some SMs and none to others (measured 4 % slower multilevel): keep the launch order
-  a.sms = ml ? 0 : sm_remap(lat);
-  const bool alternate = a.sms == 0 && alternate_order(lat);
+  const int sms = set_quad(a, lat, ml != 0);
+  const bool alternate = sms == 0 && alternate_order(lat);
   const int src = metropolis_src(lat, rng);
   const int var = sweep_variant(lat, src, ml);
   if (var == U1V_WAVE) return launch_wave(lat, links, rng, metrop, ovrn, meas_partials);
@@ -1374,7 +1399,7 @@ extern "C" int u1_update_phase(u1_lattice *lat, u1_rng *rng, int metropolis, int
   a.replay = rng->replay_dev;
   a.replay_base = rng->replay_base;
   set_proposal(a, lat);
-  a.sms = sm_remap(lat);
+  set_quad(a, lat, false);
 #ifdef U1_BOUNDS_CHECK
   a.chk = lat->ctx->chk;
   a.shadow = lat->shadow;

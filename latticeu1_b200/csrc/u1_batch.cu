@@ -96,7 +96,7 @@ __device__ __forceinline__ UpdArgs batch_args(const BatchChain &sch, const Batch
 // Four sites per thread (every chain of the launch's group has N0/2 a
 // multiple of 4), at most 128 threads per block, as k_update_quad.
 template <int D, int MU, bool MET>
-__global__ void __launch_bounds__(128, 7)
+__global__ void __launch_bounds__(128, 6)
     k_batch_update_quad(const BatchChain *__restrict__ chains, const int *__restrict__ block_chain, BatchPhase ph) {
   __shared__ BatchChain sch;
   const int blk = (int)blockIdx.x + ph.block_base;

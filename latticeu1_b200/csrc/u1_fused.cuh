@@ -41,12 +41,11 @@ static __global__ void __launch_bounds__(256) k_update_meas(const UpdArgs a, dou
 
 // Four sites per thread, 128 threads (512 sites) per block: the same work
 // items and partial slots as k_update_pair_meas.
-template <int D, int MU, bool MET, int SRC = SRC_PHILOX>
-static __global__ void __launch_bounds__(128, 7) k_update_quad_meas(const UpdArgs a, double *partials) {
+template <int D, int MU, bool MET, int SRC, int CTAS>
+static __global__ void __launch_bounds__(128, CTAS) k_update_quad_meas(const UpdArgs a, double *partials) {
   __shared__ double smem[kRedWarps * 2];
   float2 m = make_float2(0.f, 0.f);
-  const int b = a.rev ? rev_block(a, (int)blockIdx.x, (int)gridDim.x)
-                      : sm_local_block((int)blockIdx.x, (int)gridDim.x, a.sms);
+  const int b = a.rev ? rev_block(a, (int)blockIdx.x, (int)gridDim.x) : sm_local_block((int)blockIdx.x, a.order);
   update_quad_body<D, MU, MET, SRC, true>(a, 4 * (b * (int)blockDim.x + (int)threadIdx.x), &m);
   double v[2] = {(double)m.x, (double)m.y};
   block_sum<2>(v, smem);

@@ -62,6 +62,7 @@ struct u1_lattice {
   int block = 256;                 // threads per block of the phase kernels (tuned with the variant)
   int remap_block = -1;            // block size remap_sms was worked out for
   int remap_sms = 0;               // SM-local block order of the four-site kernels (0: launch order)
+  int quad_ctas = 6;               // blocks per SM of the four-site kernels (6 or 7)
   // Metropolis proposal: half-width delta (0: the reference's whole-circle
   // theta' = 2 pi u), win = delta/pi as used by the kernels, hits per link
   double delta = 0.0;

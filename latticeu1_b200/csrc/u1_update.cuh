@@ -74,6 +74,13 @@ __device__ __forceinline__ float2 staple_at(const float2 *__restrict__ lat, cons
   return cweigh(ss, c.w_ss, st, c.w_st);
 }
 
+// 1/sqrt(v) of a v near 1: rsqrtf without its treatment of subnormal arguments.
+__device__ __forceinline__ float rsqrt_unit(float v) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 // Overrelaxation of one link: U' = (conj S)^2/|S|^2 * conj U, renormalised.
 // |S| == 0 gives U' = conj U (the reference's atan2(0,0) = 0 case).  The
 // reciprocal of |S|^2 only scales U' before the renormalisation, so it is the
@@ -86,10 +93,30 @@ __device__ __forceinline__ float2 overrelax_link(float2 S, float2 U) {
     float ax = fmaf(S.x, S.x, -(S.y * S.y)) * inv;
     float ay = -2.0f * S.x * S.y * inv;
     float2 Un = make_float2(fmaf(ax, U.x, ay * U.y), fmaf(ay, U.x, -ax * U.y));
-    float r = rsqrtf(fmaf(Un.x, Un.x, Un.y * Un.y));
+    const float r = rsqrt_unit(fmaf(Un.x, Un.x, Un.y * Un.y));
     return make_float2(Un.x * r, Un.y * r);
   }
   return make_float2(U.x, -U.y);
+}
+
+// Work item of launch-order block b of G when the blocks of a single wave
+// are handed to S SMs round-robin: the blocks that share SM s (b = s, s+S,
+// s+2S, ...) get consecutive items, so neighbouring x2-planes of the
+// lattice meet in the same SM's L1.  A bijection of [0, G) for any G, S.
+// Measured on B200 at 32^4: 1.7 % faster for the four-site kernel, 2.5 %
+// slower for the two-site kernel, which therefore keeps the launch order.
+struct SmOrder {
+  int S;        // SMs (0: launch order)
+  int q, rem;   // G / S, G % S
+  FastDivK fs;  // division by S
+};
+__host__ inline SmOrder sm_order(int G, int S) {
+  return S > 0 ? SmOrder{S, G / S, G % S, make_fastdiv((uint32_t)S)} : SmOrder{0, 0, 0, make_fastdiv(1)};
+}
+__device__ __forceinline__ int sm_local_block(int b, const SmOrder &o) {
+  if (o.S <= 0) return b;
+  const int r = (int)fast_div((uint32_t)b, o.fs), s = b - r * o.S;
+  return s * o.q + min(s, o.rem) + r;
 }
 
 struct UpdArgs {
@@ -109,7 +136,8 @@ struct UpdArgs {
   int ml;                              // multilevel freeze period (0 = none)
   float win;                           // SRC_WINDOW: proposal half-width / pi (0: whole circle)
   int nhits;                           // SRC_WINDOW: Metropolis hits per link and pass
-  int sms;                             // k_update_quad: > 0 remaps the block order over this many SMs
+  SmOrder order;                       // k_update_quad: block order over the SMs of a single wave
+  int ctas;                            // k_update_quad: blocks per SM (6 or 7)
   int rev;                             // != 0: blocks take their work in reverse launch order (see rev_block)
 #ifdef U1_BOUNDS_CHECK
   struct ChkState *chk;                // checked build: violation counters (see Chk below)
@@ -207,19 +235,6 @@ __device__ __forceinline__ float2 ld1(const float2 *slab, int idx, const Chk &ck
   return __ldg(slab + idx);
 }
 
-// Work item of launch-order block b of G when the blocks of a single wave
-// are handed to S SMs round-robin: the blocks that share SM s (b = s, s+S,
-// s+2S, ...) get consecutive items, so neighbouring x2-planes of the
-// lattice meet in the same SM's L1.  A bijection of [0, G) for any G, S.
-// Measured on B200 at 32^4: 1.7 % faster for the four-site kernel, 2.5 %
-// slower for the two-site kernel, which therefore keeps the launch order.
-__device__ __forceinline__ int sm_local_block(int b, int G, int S) {
-  if (S <= 0) return b;
-  const int q = G / S, rem = G - q * S;
-  const int s = b % S, r = b / S;
-  return s * q + min(s, rem) + r;
-}
-
 // Work item of block b of G in a phase with a.rev set: the last one first.
 // A lattice larger than L2 streams every link through it in each phase;
 // consecutive phases read 7 of the same 8 (direction, parity) halves, so
@@ -313,21 +328,20 @@ __device__ __forceinline__ float2 metropolis_hits(const UpdArgs &a, uint32_t s, 
 }
 
 template <int D, int MU, bool MET, int SRC>
-__device__ __forceinline__ float2 update_one(const UpdArgs &a, int i, float2 S, float2 U,
-                                             const Philox4 *blk = nullptr) {
+__device__ __forceinline__ float2 update_link(const UpdArgs &a, int p, int i, float2 S, float2 U,
+                                              unsigned long long pass, const Philox4 *blk = nullptr) {
   if (MET) {
-    const unsigned long long pass = *a.pass_dev + (unsigned long long)a.hit;
-    if (SRC == SRC_WINDOW) return metropolis_hits<MU>(a, (uint32_t)(a.p * a.g.Vh + i), pass, S, U, blk);
+    if (SRC == SRC_WINDOW) return metropolis_hits<MU>(a, (uint32_t)(p * a.g.Vh + i), pass, S, U, blk);
     float2 Un;
     float b;
     if (SRC == SRC_REPLAY) {
-      const size_t pr = ((((size_t)(pass - a.replay_base) * 2 + a.p) * D + MU) * a.g.Vh + i) * 2;
+      const size_t pr = ((((size_t)(pass - a.replay_base) * 2 + p) * D + MU) * a.g.Vh + i) * 2;
       double sn, cs;
       sincos(a.replay[pr], &sn, &cs);
       Un = make_float2((float)cs, (float)sn);
       b = (float)a.replay[pr + 1];
     } else {
-      const uint32_t s = (uint32_t)(a.p * a.g.Vh + i);
+      const uint32_t s = (uint32_t)(p * a.g.Vh + i);
       const Philox4 r = blk ? *blk : u1_metropolis_block(s, MU, a.chain, pass, a.key0, a.key1);
       float u1;
       u1_metropolis_draws(r, s, u1, b);
@@ -339,6 +353,14 @@ __device__ __forceinline__ float2 update_one(const UpdArgs &a, int i, float2 S, 
     return (expf(dS) > b) ? Un : U;
   }
   return overrelax_link(S, U);
+}
+
+// The same in a phase kernel: parity and pass from its arguments.
+template <int D, int MU, bool MET, int SRC>
+__device__ __forceinline__ float2 update_one(const UpdArgs &a, int i, float2 S, float2 U,
+                                             const Philox4 *blk = nullptr) {
+  const unsigned long long pass = MET ? *a.pass_dev + (unsigned long long)a.hit : 0ull;
+  return update_link<D, MU, MET, SRC>(a, a.p, i, S, U, pass, blk);
 }
 
 // Body of the one-site-per-thread update of EO site i of phase (a.p, MU)
@@ -530,8 +552,19 @@ __device__ __forceinline__ void update_pair_body(const UpdArgs a, int i, float2 
 // and those steps are multiples of N0/2, so the four neighbour links along
 // x1..x3 are consecutive and 32-byte aligned: one 256-bit load serves the
 // four sites.  Steps along x0 differ per site (a shift of 0 or 1 within the
-// row, wrapping at its end), so x0-shifted neighbours are loaded per site.
-// The site decode and the steps are computed once for four sites.
+// row, wrapping at its end): a shifted quad is an aligned one moved by a link
+// (Row4).  The site decode and the steps are computed once for four sites.
+//
+// What bounds it: at 32^4 the L1 data path (65-71 % busy while x0-shifted
+// links were loaded one by one, at 32 L1 wavefronts a quad against 8 for the
+// 256-bit load) and instruction issue, about evenly, over a fixed 2.2 us of
+// launch boundary and L2 round trips.  Row4 and 32-bit offsets within a half
+// lattice took the overrelaxation phase from 5.39 to 5.07 us at 32^4 and from
+// 3.67 to 3.28 us at 24^3 x 32; with 80 registers 3.15 us there, 28.6 -> 27.8
+// at 48^4 and 97 -> 94 at 64^4.  Two phases per launch (the chains that
+// directions 0, 1 or 2, 3 couple kept in a block), tiles of 2 x 4 x 4 rows per
+// block and a walk of the half-pass in L2-sized slabs were tried and are not
+// faster: 5.1, 6.0 and 6.2 us per 32^4 of sites.
 struct Quad2 {
   float2 s[4];
 };
@@ -549,7 +582,7 @@ __device__ __forceinline__ Quad2 ld_quad(const float2 *base, int idx, const Chk 
   asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=f"(q.s[0].x), "=f"(q.s[0].y), "=f"(q.s[1].x), "=f"(q.s[1].y), "=f"(q.s[2].x), "=f"(q.s[2].y),
                  "=f"(q.s[3].x), "=f"(q.s[3].y)
-               : "l"(base + idx)
+               : "l"(reinterpret_cast<const char *>(base) + (uint32_t)((uint32_t)idx << 3))
                : "memory");
   return q;
 }
@@ -561,7 +594,7 @@ __device__ __forceinline__ Quad2 ld_quad_own(const float2 *slab, int idx, const 
     for (int s = 0; s < 4; ++s) q.s[s] = make_float2(0.f, 0.f);
     return q;
   }
-  const float2 *p = slab + idx;
+  const char *p = reinterpret_cast<const char *>(slab) + (uint32_t)((uint32_t)idx << 3);
   asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=f"(q.s[0].x), "=f"(q.s[0].y), "=f"(q.s[1].x), "=f"(q.s[1].y), "=f"(q.s[2].x), "=f"(q.s[2].y),
                  "=f"(q.s[3].x), "=f"(q.s[3].y)
@@ -571,17 +604,76 @@ __device__ __forceinline__ Quad2 ld_quad_own(const float2 *slab, int idx, const 
 }
 __device__ __forceinline__ void st_quad(float2 *slab, int idx, const float2 n[4], const Chk &ck) {
   if (!chk<4, CHK_WRITE>(ck, slab, idx)) return;
-  float2 *p = slab + idx;
+  char *p = reinterpret_cast<char *>(slab) + (uint32_t)((uint32_t)idx << 3);
   asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(n[0].x), "f"(n[0].y), "f"(n[1].x),
                "f"(n[1].y), "f"(n[2].x), "f"(n[2].y), "f"(n[3].x), "f"(n[3].y)
                : "memory");
 }
-// Per-site links at base + i + s + sh[s], s = 0..3.
-__device__ __forceinline__ Quad2 ld_shifted(const float2 *base, int i, const int sh[4], const Chk &ck) {
-  Quad2 q;
+// The x0-row a thread's four sites lie in.  A site's neighbour along x0 sits at
+// its own EO index or one further along the row: x + e0 at +1 in the rows whose
+// sites have odd x0 (`odd`), x - e0 at -1 in the others, and the step wraps at
+// the row's ends.  So a shifted quad is the aligned quad moved by one link, and
+// the one link it lacks is the first (odd) or last of the neighbouring quad of
+// the row, which the lane `src` of the warp has just loaded.
+struct Row4 {
+  bool odd;
+  int src;        // lane holding the neighbouring quad of the row
+  bool out;       // that quad belongs to another warp (N0/8 does not divide 32): load the link
+  bool any;       // some lane of the warp has `out` set
+  int edge;       // EO step from the thread's first site to that link
+  unsigned mask;  // lanes of the warp that update links (whole rows of them)
+};
+__device__ __forceinline__ Row4 row4(const GeomK &g, int x0, int k) {
+  Row4 r;
+  r.odd = (x0 & 1) != 0;
+  const int lane = (int)(threadIdx.x & 31), last = g.hN0 - 4;  // last: row offset of the last quad
+  const bool wrap = r.odd ? k == last : k == 0;
+  const int back = (last >> 2);  // lanes between the row's first and last quad
+  r.src = r.odd ? (wrap ? lane - back : lane + 1) : (wrap ? lane + back : lane - 1);
+  r.out = (unsigned)r.src > 31u;
+  r.edge = r.odd ? (wrap ? -last : 4) : (wrap ? g.hN0 - 1 : -1);
+  return r;
+}
+// The link of the neighbouring quad: `mine` is what this lane's quad lends.
+__device__ __forceinline__ float2 row4_edge(const float2 *base, int idx, const Row4 &r, float2 mine, bool used,
+                                            const Chk &ck) {
+  float2 v = make_float2(__shfl_sync(r.mask, mine.x, r.src & 31), __shfl_sync(r.mask, mine.y, r.src & 31));
+  if (r.any)
+    if (r.out && used) v = ld1(base, idx + r.edge, ck);
+  return v;
+}
+// Links at x + e0 of the sites of quad idx.
+__device__ __forceinline__ Quad2 ld_quad_fwd0(const float2 *base, int idx, const Row4 &r, const Chk &ck) {
+  Quad2 q = ld_quad(base, idx, ck);
+  const float2 v = row4_edge(base, idx, r, q.s[0], r.odd, ck);
 #pragma unroll
-  for (int s = 0; s < 4; ++s) q.s[s] = ld1(base, i + s + sh[s], ck);
+  for (int s = 0; s < 4; ++s) {
+    const float2 n = s < 3 ? q.s[s < 3 ? s + 1 : 3] : v;
+    q.s[s] = make_float2(r.odd ? n.x : q.s[s].x, r.odd ? n.y : q.s[s].y);
+  }
   return q;
+}
+// Links at x - e0 of the sites of quad idx.
+__device__ __forceinline__ Quad2 ld_quad_bwd0(const float2 *base, int idx, const Row4 &r, const Chk &ck) {
+  Quad2 q = ld_quad(base, idx, ck);
+  const float2 v = row4_edge(base, idx, r, q.s[3], !r.odd, ck);
+#pragma unroll
+  for (int s = 3; s >= 0; --s) {
+    const float2 n = s > 0 ? q.s[s > 0 ? s - 1 : 0] : v;
+    q.s[s] = make_float2(r.odd ? q.s[s].x : n.x, r.odd ? q.s[s].y : n.y);
+  }
+  return q;
+}
+// Both: the five links w[0..4] of which w[0..3] are at x - e0 and w[1..4] at x + e0.
+__device__ __forceinline__ void ld_row5(const float2 *base, int idx, const Row4 &r, float2 (&w)[5], const Chk &ck) {
+  const Quad2 q = ld_quad(base, idx, ck);
+  const float2 v = row4_edge(base, idx, r, make_float2(r.odd ? q.s[0].x : q.s[3].x, r.odd ? q.s[0].y : q.s[3].y),
+                             true, ck);
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+    const float2 o = s < 4 ? q.s[s < 4 ? s : 3] : v, e = s > 0 ? q.s[s > 0 ? s - 1 : 0] : v;
+    w[s] = make_float2(r.odd ? o.x : e.x, r.odd ? o.y : e.y);
+  }
 }
 
 // Body of the four-sites-per-thread update for EO sites i..i+3 (i a multiple
@@ -597,22 +689,21 @@ __device__ __forceinline__ void update_quad_body(const UpdArgs a, int i, float2 
   eo_decode_fast<D>(a.g, i, a.p, x, k);
   int fwd[4], bwd[4];
   eo_steps<D>(a.g, x, k, fwd, bwd);  // steps of site i; sites i+1..i+3 share those along x1..x3
-  const int odd = x[0] & 1;
-  int f0[4], b0[4];  // x0 steps of the four sites (k multiple of 4: only site 3 can end the row, site 0 start it)
-#pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    f0[s] = odd ? ((s == 3 && k + 3 == a.g.hN0 - 1) ? a.g.wrapf[0] : 1) : 0;
-    b0[s] = odd ? 0 : ((s == 0 && k == 0) ? a.g.wrapb[0] : -1);
-  }
+  Row4 row = row4(a.g, x[0], k);
+  // freeze rule, src/multilevel.cu:41 (rows lie in one time slice: they are updated or not as a whole)
+  const bool active = i < a.g.Vh && (MEAS || MU == 3 || a.ml == 0 || (x[D - 1] & (a.ml - 1)) != 0);
+  row.mask = __ballot_sync(0xffffffffu, active);
+  row.any = __any_sync(0xffffffffu, row.out);
   phase_entry<MET>(a);
-  if (i >= a.g.Vh) return;
-  if (!MEAS && MU != 3 && a.ml > 0 && (x[D - 1] & (a.ml - 1)) == 0) return;  // freeze rule, src/multilevel.cu:41
+  if (!active) return;
   const int q = 1 - a.p;
   const int V = a.g.V, Vh = a.g.Vh;
   const float2 *lat = a.lat;
   const float2 *Lq_mu = lat + MU * V + q * Vh;
   const Chk ck = make_chk(a);
   float2 ss[4], st[4], mA[4], mD[4];  // mA, mD: measurement sums (MEAS), see update_single_body
+  // the first term of each sum is stored, not added to 0 (equal up to the sign of a zero)
+  constexpr int kFirst = MU == 0 ? 1 : 0;
 #pragma unroll
   for (int s = 0; s < 4; ++s) ss[s] = st[s] = mA[s] = mD[s] = make_float2(0.f, 0.f);
 #pragma unroll
@@ -623,17 +714,22 @@ __device__ __forceinline__ void update_quad_body(const UpdArgs a, int i, float2 
     Quad2 A, B, C, Dd, E, F;
     C = ld_quad(Lp_nu, i, ck);
     if (MU == 0) {  // nu != 0: steps along nu shared, along x0 per site
-      A = ld_shifted(Lq_nu, i, f0, ck);
+      A = ld_quad_fwd0(Lq_nu, i, row, ck);
       B = ld_quad(Lq_mu, i + fwd[nu], ck);
-      Dd = ld_shifted(Lp_nu, i + bwd[nu], f0, ck);
+      Dd = ld_quad_fwd0(Lp_nu, i + bwd[nu], row, ck);
       E = ld_quad(Lq_mu, i + bwd[nu], ck);
       F = ld_quad(Lq_nu, i + bwd[nu], ck);
     } else if (nu == 0) {  // MU != 0
       A = ld_quad(Lq_nu, i + fwd[MU], ck);
-      B = ld_shifted(Lq_mu, i, f0, ck);
-      Dd = ld_shifted(Lp_nu, i + fwd[MU], b0, ck);
-      E = ld_shifted(Lq_mu, i, b0, ck);
-      F = ld_shifted(Lq_nu, i, b0, ck);
+      Dd = ld_quad_bwd0(Lp_nu, i + fwd[MU], row, ck);
+      F = ld_quad_bwd0(Lq_nu, i, row, ck);
+      float2 w[5];
+      ld_row5(Lq_mu, i, row, w, ck);
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        E.s[s] = w[s];
+        B.s[s] = w[s + 1];
+      }
     } else {  // MU != 0, nu != 0: every load 256-bit
       A = ld_quad(Lq_nu, i + fwd[MU], ck);
       B = ld_quad(Lq_mu, i + fwd[nu], ck);
@@ -646,9 +742,9 @@ __device__ __forceinline__ void update_quad_body(const UpdArgs a, int i, float2 
       const float2 up = cmulc(cmulc(A.s[s], B.s[s]), C.s[s]), lo = cmul(cconjmul(Dd.s[s], E.s[s]), F.s[s]);
       const float2 t = cadd(up, lo);
       if (MU == D - 1 || nu == D - 1)
-        st[s] = cadd(st[s], t);
+        st[s] = (MU == D - 1 ? nu == kFirst : true) ? t : cadd(st[s], t);
       else
-        ss[s] = cadd(ss[s], t);
+        ss[s] = nu == kFirst ? t : cadd(ss[s], t);
       if (MEAS && nu < MU) {
         if (MU != D - 1) mA[s] = cadd(mA[s], t);  // for MU = D-1 every nu < MU term is in st
         mD[s] = cadd(mD[s], csub(up, lo));
@@ -682,12 +778,15 @@ __device__ __forceinline__ void update_quad_body(const UpdArgs a, int i, float2 
   }
 }
 
-// Four sites per thread, at most 128 threads per block and a register budget
-// of 72, so 7 CTAs fit an SM (a 32^4 phase, 1024 CTAs, is then a single wave).
-template <int D, int MU, bool MET, int SRC>
-__global__ void __launch_bounds__(128, 7) k_update_quad(const UpdArgs a) {
-  const int b = a.rev ? rev_block(a, (int)blockIdx.x, (int)gridDim.x)
-                      : sm_local_block((int)blockIdx.x, (int)gridDim.x, a.sms);
+// Four sites per thread, at most 128 threads per block, CTAS blocks per SM:
+// 7 (72 registers) where only that many make a phase a single wave (1024
+// blocks at 32^4), 6 (80 registers) elsewhere: with more than one wave, or
+// with few blocks, the eight registers keep another load in flight (B200, us
+// per overrelaxation phase at 7 / 6 blocks: 24^3 x 32 3.29 / 3.15, 32^4 5.08 /
+// 6.04, 48^4 28.6 / 27.8, 64^4 97.1 / 93.9).
+template <int D, int MU, bool MET, int SRC, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) k_update_quad(const UpdArgs a) {
+  const int b = a.rev ? rev_block(a, (int)blockIdx.x, (int)gridDim.x) : sm_local_block((int)blockIdx.x, a.order);
   update_quad_body<D, MU, MET, SRC>(a, 4 * (b * (int)blockDim.x + (int)threadIdx.x));
 }
 

@@ -25,6 +25,7 @@
 #include "u1_internal.h"
 #include "u1_fused.cuh"
 #include "u1_wave.cuh"
+#include "u1_cluster.cuh"
 #include "u1_multilevel.cuh"
 
 using namespace u1b;
@@ -137,7 +138,7 @@ int ensure_scratch(u1_lattice *lat, size_t partial_doubles, size_t out_doubles) 
   if (partial_doubles > lat->partials_cap) {
     // cached sweep graphs hold the old scratch pointers
     cudaStreamSynchronize(lat->stream);
-    for (auto &kv : lat->graphs) cudaGraphExecDestroy(kv.second);
+    for (auto &kv : lat->graphs) cudaGraphExecDestroy(kv.second.exec);
     lat->graphs.clear();
     if (lat->partials) u1i::dev_free(lat->partials);
     lat->partials = nullptr;
@@ -297,7 +298,7 @@ static void set_coupling(u1_lattice *lat, double beta, double aniso) {
 }
 
 static void drop_graphs(u1_lattice *lat) {
-  for (auto &kv : lat->graphs) cudaGraphExecDestroy(kv.second);
+  for (auto &kv : lat->graphs) cudaGraphExecDestroy(kv.second.exec);
   lat->graphs.clear();
   if (lat->ml_g4) cudaGraphExecDestroy(lat->ml_g4);
   if (lat->ml_g2) cudaGraphExecDestroy(lat->ml_g2);
@@ -866,6 +867,76 @@ static int sweep_variant(const u1_lattice *lat, int src, int ml) {
   return v;
 }
 
+// The cluster kernel of a lattice's dimension and proposal source.
+using ClusterFn = void (*)(const UpdArgs, const ClusterK, int, int, unsigned long long *);
+template <int D>
+static ClusterFn cluster_fn_d(bool win, bool one) {
+  if (win) return one ? k_sweep_cluster<D, SRC_WINDOW, true> : k_sweep_cluster<D, SRC_WINDOW, false>;
+  return one ? k_sweep_cluster<D, SRC_PHILOX, true> : k_sweep_cluster<D, SRC_PHILOX, false>;
+}
+static ClusterFn cluster_fn(int dims, bool win, bool one) {
+  return dims == 2 ? cluster_fn_d<2>(win, one) : dims == 3 ? cluster_fn_d<3>(win, one) : cluster_fn_d<4>(win, one);
+}
+
+static cudaLaunchConfig_t cluster_config(const u1_lattice *lat, cudaLaunchAttribute *attr) {
+  const ClusterK &c = lat->cluster;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)c.blocks);
+  cfg.blockDim = dim3((unsigned)c.threads);
+  cfg.dynamicSmemBytes = (size_t)2 * lat->g.dims * c.hs * sizeof(float2);
+  cfg.stream = lat->stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)c.blocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// Whether the sweeps of `lat` run as one cluster launch (u1_cluster.cuh): a
+// lattice that fits, with an automatically chosen variant.  One block up to
+// 512 sites of a parity (its barrier costs about 0.3 us a phase, a
+// cluster's 0.6: 2D 32^2 10.4 us a sweep against 12.4), else 16 blocks
+// (8^4: 30.8 us; 8 blocks 33.1, 4 blocks 39.1; the phase kernels 71.8).  In
+// four dimensions distributed shared memory carries 19 link reads per site
+// and the gain is gone at about 700 sites per block (12^4, 648: 73.9 us
+// against 86.2), so larger 4D lattices keep the phase kernels; 2D and 3D
+// lattices use all 1024 threads (3D 32^3: 45.0 against 51.3).
+// U1_CLUSTER=0 in the environment turns it off; the checked build checks the
+// phase kernels.
+static bool cluster_usable(u1_lattice *lat, int src) {
+#ifdef U1_BOUNDS_CHECK
+  return false;
+#endif
+  if (lat->explicit_variant || src == SRC_REPLAY) return false;
+  if (lat->cluster_ok < 0) {
+    lat->cluster_ok = 0;
+    const char *env = std::getenv("U1_CLUSTER");
+    const GeomK &g = lat->g;
+    if (env && env[0] == '0') return false;
+    if (!cluster_layout(g, g.Vh <= 512 ? 1 : kClusterBlocks, lat->cluster)) return false;
+    if (g.dims == 4 && lat->cluster.threads > 704) return false;
+    const bool one = lat->cluster.blocks == 1;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cluster_config(lat, attr);
+    bool ok = true;
+    for (bool win : {false, true}) {
+      const void *fn = reinterpret_cast<const void *>(cluster_fn(g.dims, win, one));
+      ok = ok && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      2 * g.dims * kClusterThreads * (int)sizeof(float2)) == cudaSuccess;
+      ok = ok && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+      int n = 0;
+      ok = ok && cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n >= 1;
+    }
+    if (!ok) {
+      cudaGetLastError();  // not available here: the phase kernels run
+      return false;
+    }
+    lat->cluster_ok = 1;
+  }
+  return lat->cluster_ok == 1;
+}
+
 // Phase (1, MU) of the last pass with the measurement terms (u1_fused.cuh),
 // writing the per-block partials of slot MU-1 into `partials`.
 template <int D, int MU>
@@ -968,8 +1039,9 @@ static int launch_poly_finish(u1_lattice *lat, int variant, double *dev_out) {
 // meas_partials != nullptr: phases (1, mu >= 1) of the sweep's last pass run
 // as the measuring kernels, writing their partial plaquette sums there
 // (meas_sweep_scratch doubles; k_poly_finish completes the measurement).
+// phases: one launch per phase even where the lattice fits a cluster (tuning).
 static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, int ovrn, int ml,
-                       double *meas_partials = nullptr) {
+                       double *meas_partials = nullptr, bool phases = false) {
   UpdArgs a{};
   a.lat = links;
   a.g = lat->g;
@@ -987,11 +1059,21 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
   a.shadow = lat->shadow;
   a.chk_base = links;
 #endif
+  const int src = metropolis_src(lat, rng);
+  if (!phases && !meas_partials && cluster_usable(lat, src)) {
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cluster_config(lat, attr);
+    const cudaError_t e =
+        cudaLaunchKernelEx(&cfg, cluster_fn(lat->g.dims, src == SRC_WINDOW, lat->cluster.blocks == 1), (const UpdArgs)a,
+                           (const ClusterK)lat->cluster, metrop, ovrn, rng->pass_dev);
+    u1i::g_launches.fetch_add(1, std::memory_order_relaxed);
+    if (e != cudaSuccess) return u1i::cuda_fail(e, "k_sweep_cluster");
+    return U1_OK;
+  }
   // with a freeze period the SM-local order would hand whole frozen slabs to
   // some SMs and none to others (measured 4 % slower multilevel): keep the launch order
   const int sms = set_quad(a, lat, ml != 0);
   const bool alternate = sms == 0 && alternate_order(lat);
-  const int src = metropolis_src(lat, rng);
   const int var = sweep_variant(lat, src, ml);
   if (var == U1V_WAVE) return launch_wave(lat, links, rng, metrop, ovrn, meas_partials);
   const int D = lat->g.dims;
@@ -1056,12 +1138,14 @@ static int check_replay(const u1_lattice *lat, const u1_rng *rng, int metrop) {
 }
 
 // Capture `fn` (which issues work on lat->stream) into an executable graph.
+// `launches`: the kernels a replay launches.
 template <class F>
-static int capture_graph(u1_lattice *lat, F fn, cudaGraphExec_t *exec) {
+static int capture_graph(u1_lattice *lat, F fn, cudaGraphExec_t *exec, unsigned long long *launches = nullptr) {
   cudaGraph_t graph = nullptr;
   U1_CUDA_TRY(cudaStreamBeginCapture(lat->stream, cudaStreamCaptureModeThreadLocal));
   const unsigned long long launches0 = u1i::g_launches.load();
   int rc = fn();
+  if (launches) *launches = u1i::g_launches.load() - launches0;
   u1i::g_launches.store(launches0);  // captured kernels run (and count) at graph launch
   cudaError_t e = cudaStreamEndCapture(lat->stream, &graph);
   if (rc) {
@@ -1197,7 +1281,7 @@ static int tune_update(u1_lattice *lat, u1_rng *rng, bool use_cache) {
       lat->variant = vt.first;
       lat->block = vt.second;
       cudaGraphExec_t ex = nullptr;
-      rc = capture_graph(lat, [&]() { return issue_sweep(lat, lat->links, rng, 1, 4, 0); }, &ex);
+      rc = capture_graph(lat, [&]() { return issue_sweep(lat, lat->links, rng, 1, 4, 0, nullptr, true); }, &ex);
       double us = 0.0;
       if (!rc && !warmed) {
         const cudaError_t er = u1i::warm_clocks(ex, lat->stream, 50.0);
@@ -1246,6 +1330,7 @@ extern "C" int u1_tune(u1_lattice *lat, u1_rng *rng, int *variant) {
   U1_CUDA_TRY(cudaSetDevice(lat->ctx->device));
   int rc = tune_update(lat, rng, false);
   if (rc) return rc;
+  lat->explicit_variant = false;
   if (variant) *variant = lat->variant;
   return U1_OK;
 }
@@ -1255,6 +1340,7 @@ extern "C" int u1_lattice_set_variant(u1_lattice *lat, int variant) {
   if (variant != U1V_AUTO && !variant_valid(lat, variant))
     return fail(U1_ERR_INVALID, "u1_lattice_set_variant: variant not valid for this geometry (pair variants need Nx/2 even)");
   lat->variant = variant;
+  lat->explicit_variant = variant != U1V_AUTO;
   drop_graphs(lat);
   return U1_OK;
 }
@@ -1319,20 +1405,21 @@ static int update_impl(u1_lattice *lat, u1_rng *rng, int metrop, int ovrn, doubl
     rc = tune_update(lat, rng, true);
     if (rc) return rc;
   }
+  cluster_usable(lat, metropolis_src(lat, rng));  // worked out before a capture
   if (lat->use_graphs && !replay && sweep_variant(lat, metropolis_src(lat, rng), 0) != U1V_WAVE) {
     // graph key: passes, rng object, seed/chain and whether the last pass measures
     auto key = std::make_tuple(metrop * 2 + (meas_partials ? 1 : 0), ovrn, rng->id,
                                rng->seed ^ ((uint64_t)rng->chain << 48));
     auto it = lat->graphs.find(key);
     if (it == lat->graphs.end()) {
-      cudaGraphExec_t ex = nullptr;
+      SweepGraph sg;
       rc = capture_graph(lat, [&]() { return issue_sweep(lat, lat->links, rng, metrop, ovrn, 0, meas_partials); },
-                         &ex);
+                         &sg.exec, &sg.launches);
       if (rc) return rc;
-      it = lat->graphs.emplace(key, ex).first;
+      it = lat->graphs.emplace(key, sg).first;
     }
-    U1_CUDA_TRY(cudaGraphLaunch(it->second, lat->stream));
-    u1i::g_launches += (unsigned long long)(2 * lat->g.dims * (metrop + ovrn) + (ovrn == 0 ? 1 : 0));
+    U1_CUDA_TRY(cudaGraphLaunch(it->second.exec, lat->stream));
+    u1i::g_launches += it->second.launches;
   } else {
     rc = issue_sweep(lat, lat->links, rng, metrop, ovrn, 0, meas_partials);
     if (rc) return rc;
@@ -1364,6 +1451,10 @@ extern "C" int u1_update_measure(u1_lattice *lat, u1_rng *rng, int metrop, int o
   }
   int rc = u1i::ensure_scratch(lat, meas_sweep_scratch(lat->g), 8);
   if (rc) return rc;
+  if (cluster_usable(lat, metropolis_src(lat, rng))) {  // the sweep in one launch, then the measurement
+    rc = update_impl(lat, rng, metrop, ovrn, nullptr);
+    return rc ? rc : measure_dispatch(lat, dev_out);
+  }
   rc = update_impl(lat, rng, metrop, ovrn, lat->partials);
   if (rc) return rc;
   const int var = sweep_variant(lat, metropolis_src(lat, rng), 0);
@@ -1600,8 +1691,8 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
     U1_LAUNCH_CHECK("k_ml_T2");
     return U1_OK;
   };
-  const unsigned long long per_sweep = 2ull * g.dims * (metrop + ovrn) + (ovrn == 0 ? 1 : 0);
   const bool graphed = lat->use_graphs && !rng->replay_dev;
+  cluster_usable(lat, metropolis_src(lat, rng));  // worked out before a capture
   // the graphs of the last (k4, k2, metrop, ovrn, rng) are kept with the lattice
   const auto key = std::make_tuple(k4, k2, metrop, ovrn, rng->id, rng->seed ^ ((uint64_t)rng->chain << 48));
   auto body = [&]() -> int {
@@ -1614,10 +1705,10 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
       lat->ml_g4 = lat->ml_g2 = nullptr;
       lat->ml_key = std::make_tuple(-1, -1, -1, -1, (uint64_t)0, (uint64_t)0);
       if (k4 > 0) {
-        int r = capture_graph(lat, level4, &lat->ml_g4);
+        int r = capture_graph(lat, level4, &lat->ml_g4, &lat->ml_n4);
         if (r) return r;
       }
-      int r = capture_graph(lat, level2, &lat->ml_g2);
+      int r = capture_graph(lat, level2, &lat->ml_g2, &lat->ml_n2);
       if (r) return r;
       lat->ml_key = key;
     }
@@ -1626,7 +1717,7 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
       if (graphed) {
         if (k4 > 0) {
           U1_CUDA_TRY(cudaGraphLaunch(g4, lat->stream));
-          u1i::g_launches += per_sweep * (unsigned long long)k4;
+          u1i::g_launches += lat->ml_n4;
         }
       } else {
         int r = level4();
@@ -1637,7 +1728,7 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
       for (int k = 0; k < n2; ++k) {
         if (graphed) {
           U1_CUDA_TRY(cudaGraphLaunch(g2, lat->stream));
-          u1i::g_launches += per_sweep * (unsigned long long)k2 + 2ull;
+          u1i::g_launches += lat->ml_n2;
         } else {
           int r = level2();
           if (r) return r;

@@ -12,6 +12,17 @@
 #include "u1_geom.cuh"
 
 namespace u1b {
+// Layout of a sweep in one thread-block cluster (u1_cluster.cuh).
+struct ClusterK {
+  int blocks;   // blocks of the cluster
+  int rows;     // x0-rows per block
+  int hs;       // links of one (direction, parity) a block holds: rows * N0/2
+  int threads;  // threads per block
+  FastDivK fr;  // division by rows
+};
+}  // namespace u1b
+
+namespace u1b {
 struct ChkState;
 }
 
@@ -37,6 +48,12 @@ struct u1_rng {
 // Update kernel variants (all bit-identical; the tuner picks the fastest).
 enum : int { U1V_AUTO = 0, U1V_PAIR32 = 1, U1V_PAIR = 2, U1V_SINGLE = 3, U1V_WAVE = 4, U1V_QUAD = 5 };
 
+// A captured sweep and the kernels one replay of it launches.
+struct SweepGraph {
+  cudaGraphExec_t exec = nullptr;
+  unsigned long long launches = 0;
+};
+
 struct u1_lattice {
   u1_ctx *ctx = nullptr;
   cudaStream_t stream = nullptr;
@@ -56,10 +73,13 @@ struct u1_lattice {
   double *stage = nullptr;          // FP64 angle staging buffer for host import/export (V*dims)
   cudaStream_t own_stream = nullptr; // used when no stream is attached
   // cached CUDA graphs of whole sweeps, keyed by (metrop, ovrn, rng id, seed)
-  std::map<std::tuple<int, int, uint64_t, uint64_t>, cudaGraphExec_t> graphs;
+  std::map<std::tuple<int, int, uint64_t, uint64_t>, SweepGraph> graphs;
   bool use_graphs = true;
   int variant = U1V_AUTO;          // update kernel variant (U1V_AUTO: tune on first update)
   int block = 256;                 // threads per block of the phase kernels (tuned with the variant)
+  bool explicit_variant = false;   // set by u1_lattice_set_variant (else chosen automatically)
+  int cluster_ok = -1;             // sweeps as one cluster launch: -1 unknown, 0 no, 1 yes (layout: cluster)
+  u1b::ClusterK cluster{};
   int remap_block = -1;            // block size remap_sms was worked out for
   int remap_sms = 0;               // SM-local block order of the four-site kernels (0: launch order)
   int quad_ctas = 6;               // blocks per SM of the four-site kernels (6 or 7)
@@ -79,6 +99,7 @@ struct u1_lattice {
   double2 *ml_P2 = nullptr, *ml_T2 = nullptr, *ml_T4 = nullptr;
   std::tuple<int, int, int, int, uint64_t, uint64_t> ml_key{-1, -1, -1, -1, 0, 0};
   cudaGraphExec_t ml_g4 = nullptr, ml_g2 = nullptr;
+  unsigned long long ml_n4 = 0, ml_n2 = 0;  // kernels per replay
   unsigned wave_spin_limit = 0;    // polls per neighbour wait (0: the kernel's default)
   int wave_stall_tile = -1;        // test hook: this tile never publishes its phases (-1: none)
   unsigned *shadow = nullptr;      // checked build: per-link access marks (V*dims words)

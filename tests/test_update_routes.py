@@ -1,0 +1,89 @@
+"""Routes a sweep can take: the four-site kernel at rows that do and do not
+divide a warp, and the one-launch cluster sweep of small lattices, against the
+one-site kernel.  All routes do the same arithmetic in the same order, so the
+links are compared bit for bit."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from latticeu1_b200 import Context
+    return Context(0)
+
+
+def _chain(ctx, dims, N, aniso, variant, block=0, window=None, sweeps=((1, 2), (2, 0), (0, 1))):
+    import torch
+
+    from latticeu1_b200 import Lattice, Rng
+    lat = Lattice(ctx, dims, N, 1.1, aniso)
+    if variant:
+        lat.set_variant(variant)
+    if block:
+        lat.set_block(block)
+    if window:
+        lat.set_metropolis(*window)
+    rng = Rng(ctx, 31)
+    lat.hot_start(rng)
+    for m, o in sweeps:
+        lat.update(rng, m, o)
+    obs = torch.zeros(6, dtype=torch.float64, device="cuda")
+    lat.update_measure(rng, 1, 1, obs.data_ptr())
+    torch.cuda.synchronize()
+    out = lat.export_angles(), obs.cpu().numpy().copy(), rng.state
+    ref = lat.measure()
+    lat.close()
+    flat = np.array([f(ref[k]) for k in ("plaq_ss", "plaq_st", "poly") for f in (np.real, np.imag)])
+    # the measurement of the same links, summed in FP64 from FP32 terms of a few sites
+    assert np.nanmax(np.abs(out[1] - flat)) < 1e-6  # 2D has no spatial plaquettes: NaN
+    return out
+
+
+# x0-rows of 1, 2, 3, 5, 6, 8, 12 and 33 quads: within a warp, across warps,
+# longer than a warp; the last block partly filled
+@pytest.mark.parametrize("dims,N", [
+    (4, (8, 6, 4, 6)), (4, (16, 4, 6, 4)), (4, (24, 4, 4, 6)), (4, (40, 6, 4, 4)), (4, (48, 4, 6, 4)),
+    (3, (64, 6, 0, 10)), (3, (96, 4, 0, 6)), (2, (264, 0, 0, 6))])
+@pytest.mark.parametrize("block", [64, 128])
+def test_four_site_rows(ctx, dims, N, block):
+    a = _chain(ctx, dims, N, 1.5, 5, block)
+    b = _chain(ctx, dims, N, 1.5, 3)
+    assert np.array_equal(a[0], b[0]) and a[2] == b[2]
+
+
+# one block (up to 512 sites of a parity) and sixteen, shares that do not divide
+# the rows (idle and short blocks), the smallest extents, the largest lattices
+# of the route and the first ones beyond it
+@pytest.mark.parametrize("dims,N", [
+    (2, (4, 0, 0, 4)), (2, (32, 0, 0, 32)), (2, (34, 0, 0, 32)), (2, (62, 0, 0, 46)), (2, (128, 0, 0, 256)),
+    (2, (130, 0, 0, 256)), (2, (2048, 0, 0, 16)), (3, (2, 2, 0, 2)), (3, (10, 6, 0, 14)), (3, (32, 32, 0, 32)),
+    (4, (2, 2, 2, 2)), (4, (8, 8, 8, 2)), (4, (6, 10, 8, 4)), (4, (8, 8, 8, 8)), (4, (10, 12, 14, 12)),
+    (4, (22, 8, 8, 16)), (4, (22, 8, 16, 8))])
+@pytest.mark.parametrize("window", [None, (0.7, 3)])
+def test_cluster_sweep(ctx, dims, N, window, monkeypatch):
+    monkeypatch.setenv("U1_TUNE", "0")
+    a = _chain(ctx, dims, N, 0.8, 0, window=window)
+    b = _chain(ctx, dims, N, 0.8, 3, window=window)
+    assert np.array_equal(a[0], b[0]) and a[2] == b[2]
+
+
+def test_cluster_sweep_in_multilevel(ctx, monkeypatch):
+    """Frozen time slices, the work copy of the links, graphs on and off."""
+    from latticeu1_b200 import Lattice, Rng
+    monkeypatch.setenv("U1_TUNE", "0")
+    res = []
+    for variant, graphs in ((0, True), (0, False), (3, True)):
+        lat = Lattice(ctx, 4, (6, 4, 8, 12), 0.95)
+        if variant:
+            lat.set_variant(variant)
+        lat.set_graphs(graphs)
+        rng = Rng(ctx, 3)
+        lat.hot_start(rng)
+        res.append((lat.multilevel(rng, 2, 1, 3, 2, 1, 2), lat.export_angles(), rng.state))
+        lat.close()
+    for r in res[1:]:
+        assert np.array_equal(r[0], res[0][0]) and np.array_equal(r[1], res[0][1]) and r[2] == res[0][2]

@@ -1553,9 +1553,8 @@ extern "C" int u1_measure(u1_lattice *lat, double out[6]) {
   if (rc) return rc;
   rc = u1i::ensure_scratch(lat, 0, 8);
   if (rc) return rc;
-  rc = measure_dispatch(lat, nullptr);
+  rc = measure_dispatch(lat, lat->h_out);  // pinned host memory: the kernel stores its six results there itself
   if (rc) return rc;
-  U1_CUDA_TRY(cudaMemcpyAsync(lat->h_out, lat->d_out, 6 * sizeof(double), cudaMemcpyDeviceToHost, lat->stream));
   U1_CUDA_TRY(cudaStreamSynchronize(lat->stream));
   memcpy(out, lat->h_out, 6 * sizeof(double));
   return U1_OK;
@@ -1582,11 +1581,11 @@ extern "C" int u1_polyakov(u1_lattice *lat, double out[2]) {
 
 template <int D>
 static int launch_poly_field(u1_lattice *lat, const float2 *links, int multihit) {
-  const int nb = u1i::blocks_for(lat->g.Vs, 256);
+  const int nb = u1i::blocks_for(lat->g.Vs, 32);
   if (multihit)
-    k_poly_field<D, true><<<nb, 256, 0, lat->stream>>>(links, lat->g, lat->c, lat->pfield);
+    k_poly_field<D, true><<<nb, 32 * kPolyWarps, 0, lat->stream>>>(links, lat->g, lat->c, lat->pfield);
   else
-    k_poly_field<D, false><<<nb, 256, 0, lat->stream>>>(links, lat->g, lat->c, lat->pfield);
+    k_poly_field<D, false><<<nb, 32 * kPolyWarps, 0, lat->stream>>>(links, lat->g, lat->c, lat->pfield);
   U1_LAUNCH_CHECK("k_poly_field");
   return U1_OK;
 }
@@ -1598,7 +1597,7 @@ extern "C" int u1_poly_corr(u1_lattice *lat, int multihit, double *out, int out_
   if (out_len < 2 * R) return fail(U1_ERR_INVALID, "u1_poly_corr: out_len < 2*R (R = Grid[0]/2)");
   U1_CUDA_TRY(cudaSetDevice(lat->ctx->device));
   if (!lat->pfield) U1_CUDA_TRY(u1i::dev_alloc(&lat->pfield, (size_t)lat->g.Vs * sizeof(double2)));
-  const int nb = u1i::blocks_for(lat->g.Vs, kRedThreads);
+  const int nb = u1i::blocks_for(lat->g.Vs, kCorrSites);
   int rc = u1i::ensure_scratch(lat, (size_t)nb * 2 * R, (size_t)2 * R);
   if (rc) return rc;
   switch (lat->g.dims) {
@@ -1609,10 +1608,8 @@ extern "C" int u1_poly_corr(u1_lattice *lat, int multihit, double *out, int out_
   if (rc) return rc;
   const double norm = 1.0 / ((double)lat->g.Vs * lat->g.tdir);
   k_poly_corr<<<nb, kRedThreads, 0, lat->stream>>>(lat->pfield, lat->g, R, lat->partials, lat->counter,
-                                                   lat->d_out, norm);
+                                                   lat->h_out, norm);
   U1_LAUNCH_CHECK("k_poly_corr");
-  U1_CUDA_TRY(cudaMemcpyAsync(lat->h_out, lat->d_out, (size_t)2 * R * sizeof(double), cudaMemcpyDeviceToHost,
-                              lat->stream));
   U1_CUDA_TRY(cudaStreamSynchronize(lat->stream));
   memcpy(out, lat->h_out, (size_t)2 * R * sizeof(double));
   return U1_OK;
@@ -1636,14 +1633,23 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
   const int nl2 = g.N[g.tdir] / 2, nl4 = g.N[g.tdir] / 4;
   int rc = U1_OK;
   auto cleanup = [&]() { cudaStreamSynchronize(lat->stream); };
-  // The work buffers (the links' working copy, slab products, T2, T4: about
-  // 210 MB at 24^3 x 32) are allocated by the first call and kept with the
-  // lattice, so later calls neither allocate nor synchronise the device.
+  // The work buffers (the links' working copy, the slab products of a batch of
+  // sub-updates, T2, T4: about 260 MB at 24^3 x 32) are allocated by the first
+  // call and kept with the lattice, so later calls neither allocate nor
+  // synchronise the device.  A batch is up to 16 sub-updates or 256 MiB of slab
+  // products; one sub-update where the device has no memory for a large batch.
   if (!lat->ml_work) {
     float2 *work = nullptr;
     double2 *P2 = nullptr, *T2 = nullptr, *T4 = nullptr;
     cudaError_t e = u1i::dev_alloc(&work, (size_t)g.V * g.dims * sizeof(float2));
-    if (e == cudaSuccess) e = u1i::dev_alloc(&P2, (size_t)g.Vs * nl2 * sizeof(double2));
+    const size_t slab_bytes = (size_t)g.Vs * nl2 * sizeof(double2);
+    int batch = (int)std::max<size_t>(1, std::min<size_t>(16, (256ull << 20) / slab_bytes));
+    if (e == cudaSuccess) e = u1i::dev_alloc(&P2, slab_bytes * batch);
+    if (e == cudaErrorMemoryAllocation && work && slab_bytes * batch > (32ull << 20) && batch > 1) {
+      cudaGetLastError();
+      batch = 1;
+      e = u1i::dev_alloc(&P2, slab_bytes);
+    }
     if (e == cudaSuccess) e = u1i::dev_alloc(&T2, size * nl2 * sizeof(double2));
     if (e == cudaSuccess) e = u1i::dev_alloc(&T4, size * nl4 * sizeof(double2));
     if (e != cudaSuccess) {
@@ -1656,6 +1662,7 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
     }
     lat->ml_work = work;
     lat->ml_P2 = P2;
+    lat->ml_batch = batch;
     lat->ml_T2 = T2;
     lat->ml_T4 = T4;
   }
@@ -1669,8 +1676,8 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
     return rc;
   }
   // The level-4 update (k4 sweeps, freeze period 4) and one level-2
-  // sub-update (k2 sweeps with freeze period 2, the multihit field, the T2
-  // accumulation) are each captured once as a CUDA graph and replayed; the
+  // sub-update's k2 sweeps (freeze period 2) are each captured once as a CUDA
+  // graph and replayed; the
   // Metropolis pass counter lives in device memory, so replays draw fresh
   // numbers exactly as direct launches would.
   auto level4 = [&]() -> int {
@@ -1685,9 +1692,23 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
       int r = issue_sweep(lat, work, rng, metrop, ovrn, 2);
       if (r) return r;
     }
-    k_ml_slab2<<<u1i::blocks_for((long long)g.Vs * nl2, 256), 256, 0, lat->stream>>>(work, g, lat->c, md, P2);
+    return U1_OK;
+  };
+  // the slab products of sub-update k of a level-4 step into their place in the
+  // batch; the batch into T2 when it is full or the last
+  const size_t slab = (size_t)g.Vs * nl2;
+  const MlLines ml = ml_lines(md);
+  auto accumulate = [&](int k) -> int {
+    const int slot = k % lat->ml_batch;
+    k_ml_slab2<<<u1i::blocks_for(g.Vs, 32) * u1i::blocks_for(2 * nl2, kSlabWarps), 32 * kSlabWarps, 0, lat->stream>>>(
+        work, g, lat->c, md, P2 + slab * slot);
     U1_LAUNCH_CHECK("k_ml_slab2");
-    k_ml_T2<<<u1i::blocks_for((long long)(size / 2) * nl2, 256), 256, 0, lat->stream>>>(P2, md, T2);
+    if (slot + 1 < lat->ml_batch && k + 1 < n2) return U1_OK;
+    const int blocks = ml.blocks * 3 * u1i::blocks_for(R, kT2R) * nl2, fresh = k < lat->ml_batch ? 1 : 0;
+    if (ml.fits)
+      k_ml_T2<false><<<blocks, ml.threads, 0, lat->stream>>>(P2, slab, slot + 1, md, ml, fresh, T2);
+    else
+      k_ml_T2<true><<<blocks, ml.threads, 0, lat->stream>>>(P2, slab, slot + 1, md, ml, fresh, T2);
     U1_LAUNCH_CHECK("k_ml_T2");
     return U1_OK;
   };
@@ -1698,7 +1719,6 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
   auto body = [&]() -> int {
     U1_CUDA_TRY(cudaMemcpyAsync(work, lat->links, (size_t)g.V * g.dims * sizeof(float2),
                                 cudaMemcpyDeviceToDevice, lat->stream));
-    U1_CUDA_TRY(cudaMemsetAsync(T4, 0, size * nl4 * sizeof(double2), lat->stream));
     if (graphed && (!lat->ml_g2 || lat->ml_key != key)) {
       if (lat->ml_g4) cudaGraphExecDestroy(lat->ml_g4);
       if (lat->ml_g2) cudaGraphExecDestroy(lat->ml_g2);
@@ -1724,7 +1744,6 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
         if (r) return r;
       }
       rng->pass += (uint64_t)metrop * (uint64_t)k4;
-      U1_CUDA_TRY(cudaMemsetAsync(T2, 0, size * nl2 * sizeof(double2), lat->stream));
       for (int k = 0; k < n2; ++k) {
         if (graphed) {
           U1_CUDA_TRY(cudaGraphLaunch(g2, lat->stream));
@@ -1733,17 +1752,17 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
           int r = level2();
           if (r) return r;
         }
+        int r = accumulate(k);
+        if (r) return r;
         rng->pass += (uint64_t)metrop * (uint64_t)k2;
       }
       k_ml_T4<<<u1i::blocks_for((long long)(size / 2) * nl4, 256), 256, 0, lat->stream>>>(T2, md, 1.0 / (double)n2,
-                                                                                        T4);
+                                                                                        i == 0 ? 1 : 0, T4);
       U1_LAUNCH_CHECK("k_ml_T4");
     }
-    k_ml_final<<<nb_s, kRedThreads, 0, lat->stream>>>(T4, g, R, 1.0 / (double)n4, lat->partials, lat->counter,
-                                                      lat->d_out, 1.0 / ((double)g.Vs * g.tdir));
+    k_ml_final<<<dim3((unsigned)nb_s, (unsigned)R), kRedThreads, 0, lat->stream>>>(
+        T4, g, R, 1.0 / (double)n4, lat->partials, lat->counter, lat->h_out, 1.0 / ((double)g.Vs * g.tdir));
     U1_LAUNCH_CHECK("k_ml_final");
-    U1_CUDA_TRY(cudaMemcpyAsync(lat->h_out, lat->d_out, (size_t)2 * R * sizeof(double),
-                                cudaMemcpyDeviceToHost, lat->stream));
     U1_CUDA_TRY(cudaStreamSynchronize(lat->stream));
     return U1_OK;
   };

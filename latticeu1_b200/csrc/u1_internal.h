@@ -96,6 +96,7 @@ struct u1_lattice {
   // T2 and T4, kept from the first call until the lattice is destroyed, and
   // the level-4 / level-2 graphs of the last (k4, k2, metrop, ovrn, rng) used
   float2 *ml_work = nullptr;
+  int ml_batch = 1;                // sub-updates whose slab products ml_P2 holds
   double2 *ml_P2 = nullptr, *ml_T2 = nullptr, *ml_T4 = nullptr;
   std::tuple<int, int, int, int, uint64_t, uint64_t> ml_key{-1, -1, -1, -1, 0, 0};
   cudaGraphExec_t ml_g4 = nullptr, ml_g2 = nullptr;

@@ -323,100 +323,152 @@ __device__ __forceinline__ float bessel_ratio_i1_i0(float x) {
   return r;
 }
 
-// Analytic multihit mean of the temporal link at site x (parity p, EO index
-// i): conj(S) * I1(beta|S|) / (|S| I0(beta|S|)).
-template <int D>
-__device__ __forceinline__ float2 multihit_link(const float2 *__restrict__ lat, const GeomK &g,
-                                                const CoupK &c, const int x[4], int i, int p) {
-  const float2 S = staple_at<D>(lat, g, c, x, i, p, g.tdir);
+// Analytic multihit mean of the temporal link whose staple is S:
+// conj(S) * I1(beta|S|) / (|S| I0(beta|S|)).
+__device__ __forceinline__ float2 multihit_mean(const CoupK &c, float2 S) {
   const float alpha = sqrtf(fmaf(S.x, S.x, S.y * S.y));
   if (!(alpha > 0.f)) return make_float2(0.f, 0.f);
   const float t = bessel_ratio_i1_i0(c.beta * alpha) / alpha;
   return make_float2(t * S.x, -t * S.y);
 }
 
-// Spatial lexicographic index s -> x[0..tdir-1] (reference indexIdS /
-// indexNOSD, include/index.h:19-24,80-84).
-__device__ __forceinline__ void spatial_decode(const GeomK &g, int s, int x[4]) {
-  x[0] = x[1] = x[2] = x[3] = 0;
-  int r = s;
-  for (int k = 0; k < g.tdir; ++k) {
-    x[k] = r % g.N[k];
-    r /= g.N[k];
+// One spatial site's column of temporal links.  The two spatial sites 2k and
+// 2k + 1 of a row share the EO index i0 on the t = 0 slice; the one of parity q
+// sits at EO index i0 + t es of parity (q + t) mod 2, and its spatial neighbour
+// steps are those of t = 0 throughout.  Threads with consecutive i0 and one q
+// read consecutive links.
+template <int D>
+struct TimeColumn {
+  int i0, q;
+  int s;  // spatial lexicographic index
+  int fwd[4], bwd[4];
+};
+template <int D>
+__device__ __forceinline__ TimeColumn<D> time_column(const GeomK &g, int col) {  // col < Vs
+  TimeColumn<D> tc;
+  const int hs = g.Vs / 2;
+  tc.q = col >= hs ? 1 : 0;
+  tc.i0 = col - tc.q * hs;
+  int x[4], k;
+  eo_decode_fast<D>(g, tc.i0, tc.q, x, k);
+  eo_steps<D>(g, x, k, tc.fwd, tc.bwd);
+  tc.s = 2 * tc.i0 + (x[0] & 1);  // rows of N0 sites are rows of N0/2 EO indices
+  return tc;
+}
+// The temporal link (MH: its multihit mean) of the column at time t.
+template <int D, bool MH>
+__device__ __forceinline__ float2 column_link(const float2 *__restrict__ lat, const GeomK &g, const CoupK &c,
+                                              const TimeColumn<D> &tc, int t) {
+  const int p = (tc.q + t) & 1, i = tc.i0 + t * g.es[D - 1];
+  if (!MH) return __ldg(lat + (size_t)(D - 1) * g.V + (size_t)p * g.Vh + i);
+  int fwd[4], bwd[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    fwd[k] = tc.fwd[k];
+    bwd[k] = tc.bwd[k];
   }
+  fwd[D - 1] = t == g.N[D - 1] - 1 ? g.wrapf[D - 1] : g.es[D - 1];
+  bwd[D - 1] = t == 0 ? g.wrapb[D - 1] : -g.es[D - 1];
+  return multihit_mean(c, staple_steps<D, D - 1>(lat, g, c, i, p, fwd, bwd, no_chk()));
 }
 
 // P(x) = prod_t U_t(x,t) (or of the multihit means) for every spatial site,
-// stored in spatial lexicographic order; products in FP64.
+// stored in spatial lexicographic order; products in FP64.  A block takes 32
+// columns and splits time over its 16 warps, whose products are then multiplied
+// in time order.  A multihit link is a chain of about 20 dependent divisions
+// after its staple, so the kernel lives on threads in flight: at 24^3 x 32 one
+// thread per column (54 blocks) took 89 us.
+constexpr int kPolyWarps = 16;
 template <int D, bool MH>
-static __global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(32 * kPolyWarps)
     k_poly_field(const float2 *__restrict__ lat, GeomK g, CoupK c, double2 *P) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= g.Vs) return;
-  int x[4];
-  spatial_decode(g, s, x);
+  __shared__ double2 part[kPolyWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int col = blockIdx.x * 32 + lane;
+  const int Nt = g.N[D - 1], per = (Nt + kPolyWarps - 1) / kPolyWarps;
+  const TimeColumn<D> tc = time_column<D>(g, min(col, g.Vs - 1));
   double2 prod = make_double2(1.0, 0.0);
-  const int Nt = g.N[g.tdir];
-  for (int t = 0; t < Nt; ++t) {
-    int y[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) y[k] = (k == g.tdir) ? t : x[k];
-    const int i = eo_index(g, y);
-    const int p = (y[0] + y[1] + y[2] + y[3]) & 1;
-    float2 u;
-    if (MH)
-      u = multihit_link<D>(lat, g, c, y, i, p);
-    else
-      u = __ldg(lat + (size_t)g.tdir * g.V + (size_t)p * g.Vh + i);
+  for (int t = w * per; t < min(Nt, (w + 1) * per); ++t) {
+    const float2 u = column_link<D, MH>(lat, g, c, tc, t);
     prod = zmul(prod, make_double2((double)u.x, (double)u.y));
   }
-  P[s] = prod;
+  part[w][lane] = prod;
+#pragma unroll
+  for (int o = 1; o < kPolyWarps; o <<= 1) {
+    __syncthreads();
+    if ((w & (2 * o - 1)) == 0) part[w][lane] = prod = zmul(prod, part[w + o][lane]);
+  }
+  if (w == 0 && col < g.Vs) P[tc.s] = prod;
 }
 
-// C(r) = norm * sum_x sum_{i<d-1} P(x) conj(P(x + r e_i)), r = 1..R.
+// Sums of partials[b * n + k] over blocks b < nb, a warp per k: out[k] = norm * sum.
+// Called by every thread of the last block to finish.
+__device__ __forceinline__ void finish_columns(const double *partials, int nb, int n, double *out, double norm) {
+  const int lane = threadIdx.x & 31;
+  for (int k = threadIdx.x >> 5; k < n; k += (int)(blockDim.x >> 5)) {
+    double v = 0.0;
+#pragma unroll 4
+    for (int b = lane; b < nb; b += 32) v += __ldcg(partials + (size_t)b * n + k);
+    v = warp_sum(v);
+    if (lane == 0) out[k] = v * norm;
+  }
+}
+
+// Whether this block is the last of `blocks` to get here; its threads then see
+// every block's partials.
+__device__ __forceinline__ bool last_block(unsigned int *counter, unsigned int blocks) {
+  __shared__ bool am_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) am_last = (atomicAdd(counter, 1u) == blocks - 1);
+  __syncthreads();
+  if (am_last) __threadfence();
+  return am_last;
+}
+
+// C(r) = norm * sum_x sum_{i<d-1} P(x) conj(P(x + r e_i)), r = 1..R.  A block
+// takes kCorrSites sites, a warp one r at a time (no block-wide reduction per
+// r: with one, 54 blocks of 256 sites took 36 us at 24^3 x 32).
 // partials: gridDim.x * 2R doubles; out: 2R doubles.
+constexpr int kCorrSites = 64;
 static __global__ void __launch_bounds__(kRedThreads)
     k_poly_corr(const double2 *__restrict__ P, GeomK g, int R, double *partials,
                 unsigned int *counter, double *out, double norm) {
-  __shared__ double smem[kRedWarps * 2];
-  __shared__ bool am_last;
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  int x[4];
-  double2 P0 = make_double2(0.0, 0.0);
-  if (s < g.Vs) {
-    spatial_decode(g, s, x);
-    P0 = P[s];
-  }
-  for (int r = 1; r <= R; ++r) {
-    double v[2] = {0.0, 0.0};
-    if (s < g.Vs) {
-      for (int dir = 0; dir < g.tdir; ++dir) {
-        int sp = 0, stride = 1;
-        for (int k = 0; k < g.tdir; ++k) {
-          int xk = x[k];
-          if (k == dir) xk = (xk + r) % g.N[k];
-          sp += xk * stride;
-          stride *= g.N[k];
-        }
-        double2 q = zmulc(P0, P[sp]);
-        v[0] += q.x;
-        v[1] += q.y;
-      }
+  const int lane = threadIdx.x & 31;
+  int x[2][3], s[2];
+  double2 P0[2];
+  int step[3] = {1, g.N[0], g.N[0] * g.N[1]};
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    s[e] = blockIdx.x * kCorrSites + 32 * e + lane;
+    const bool in = s[e] < g.Vs;
+    int r = in ? s[e] : 0;
+    P0[e] = in ? P[r] : make_double2(0.0, 0.0);
+    s[e] = r;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      x[e][k] = k < g.tdir ? r % g.N[k] : 0;
+      r = k < g.tdir ? r / g.N[k] : r;
     }
-    block_sum<2>(v, smem);
-    if (threadIdx.x < 2) partials[(size_t)blockIdx.x * 2 * R + 2 * (r - 1) + threadIdx.x] = v[0];
   }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) am_last = (atomicAdd(counter, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  for (int k = 0; k < 2 * R; ++k) {
-    double w[1] = {strided_partial_sum(partials, gridDim.x, 2 * R, k)};
-    block_sum<1>(w, smem);
-    if (threadIdx.x == 0) out[k] = w[0] * norm;
+  for (int r = 1 + (int)(threadIdx.x >> 5); r <= R; r += kRedWarps) {
+    double2 v = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (k < g.tdir) {
+        const int rk = r % g.N[k];  // r may exceed the extent of a direction other than x0
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int xk = x[e][k] + rk, d = xk >= g.N[k] ? rk - g.N[k] : rk;
+          v = zadd(v, zmulc(P0[e], P[s[e] + d * step[k]]));
+        }
+      }
+    v.x = warp_sum(v.x);
+    v.y = warp_sum(v.y);
+    if (lane == 0) *reinterpret_cast<double2 *>(partials + (size_t)blockIdx.x * 2 * R + 2 * (r - 1)) = v;
   }
+  if (!last_block(counter, gridDim.x)) return;
+  finish_columns(partials, (int)gridDim.x, 2 * R, out, norm);
   if (threadIdx.x == 0) *counter = 0u;
 }
 

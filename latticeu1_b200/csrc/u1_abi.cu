@@ -26,6 +26,7 @@
 #include "u1_fused.cuh"
 #include "u1_wave.cuh"
 #include "u1_cluster.cuh"
+#include "u1_duo.cuh"
 #include "u1_multilevel.cuh"
 
 using namespace u1b;
@@ -754,6 +755,38 @@ static int set_quad(UpdArgs &a, u1_lattice *lat, bool plain) {
   return sms;
 }
 
+// Phases (a.p, A) and (a.p, A + 1) as one launch (u1_duo.cuh).
+template <int D, int A>
+static int launch_duo_a(const UpdArgs &a, const DuoK &d, cudaStream_t s, bool met, int src) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)d.blocks);
+  cfg.blockDim = dim3((unsigned)d.threads);
+  cfg.dynamicSmemBytes = (size_t)d.threads * sizeof(float2);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = !met ? cudaLaunchKernelEx(&cfg, k_update_duo<D, A, false, SRC_PHILOX>, a, d)
+                        : src == SRC_WINDOW ? cudaLaunchKernelEx(&cfg, k_update_duo<D, A, true, SRC_WINDOW>, a, d)
+                                            : cudaLaunchKernelEx(&cfg, k_update_duo<D, A, true, SRC_PHILOX>, a, d);
+  u1i::g_launches.fetch_add(1, std::memory_order_relaxed);
+  if (e != cudaSuccess) return u1i::cuda_fail(e, "k_update_duo");
+  return U1_OK;
+}
+static int launch_duo(int dims, int A, const UpdArgs &a, const DuoK &d, cudaStream_t s, bool met, int src) {
+  if (dims == 3) return launch_duo_a<3, 0>(a, d, s, met, src);
+  return A == 0 ? launch_duo_a<4, 0>(a, d, s, met, src) : launch_duo_a<4, 2>(a, d, s, met, src);
+}
+
+// Whether a sweep at the lattice's block size can run phases two at a time
+// (3D: directions 0, 1; 4D: also 2, 3 where their chains are short).
+static bool duo_fits(const u1_lattice *lat) {
+  DuoK d;
+  return lat->g.dims >= 3 && duo_layout(lat->g, 0, lat->block, d);
+}
+
 // The proposal settings of `lat` into the kernel arguments.
 static void set_proposal(UpdArgs &a, const u1_lattice *lat) {
   a.win = lat->win;
@@ -1079,7 +1112,27 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
   const int D = lat->g.dims;
   const int total = 2 * D * (metrop + ovrn);
   int phase = 0;
+  // two phases per launch: an automatically tuned lattice whose tuner found it fastest
+  DuoK duo[2];
+  bool pair_up[2] = {false, false};
+  if (lat->duo && src != SRC_REPLAY && D >= 3) {
+    pair_up[0] = duo_layout(lat->g, 0, lat->block, duo[0]);
+    pair_up[1] = D == 4 && duo_layout(lat->g, 2, lat->block, duo[1]);
+  }
+  // Launches the phase (a.p, a.mu) or, with it, the next direction's; advances
+  // a.mu to the last direction done.
   auto launch = [&](bool met) -> int {
+    if ((a.mu & 1) == 0 && a.mu < 3 && pair_up[a.mu / 2] &&
+        !(meas_partials && phase >= total - 2 * D && a.p == 1)) {  // not where the last pass measures
+      phase += 2;
+      a.rev = 0;
+      int rc = launch_duo(D, a.mu, a, duo[a.mu / 2], lat->stream, met, src);
+      ++a.mu;
+#ifdef U1_BOUNDS_CHECK
+      if (rc == U1_OK) rc = u1i::chk_phase_end(lat->stream, a.shadow, (size_t)D * lat->g.V, a.chk);
+#endif
+      return rc;
+    }
     ++phase;
     a.rev = (alternate && (phase & 1) == 0) ? 1 : 0;  // every second phase runs its blocks backwards
     int rc;
@@ -1099,9 +1152,8 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
   };
   for (int m = 0; m < metrop; ++m)
     for (int p = 0; p < 2; ++p)
-      for (int mu = 0; mu < D; ++mu) {
+      for (a.mu = 0; a.mu < D; ++a.mu) {
         a.p = p;
-        a.mu = mu;
         a.hit = m;
         int rc = launch(true);
         if (rc) return rc;
@@ -1109,9 +1161,8 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
   bool bumped = (metrop == 0);
   for (int o = 0; o < ovrn; ++o)
     for (int p = 0; p < 2; ++p)
-      for (int mu = 0; mu < D; ++mu) {
+      for (a.mu = 0; a.mu < D; ++a.mu) {
         a.p = p;
-        a.mu = mu;
         a.hit = 0;
         a.bump_ptr = bumped ? nullptr : rng->pass_dev;
         a.bump_by = (unsigned)metrop;
@@ -1179,10 +1230,14 @@ static bool block_valid(int threads) { return threads >= 32 && threads <= 256 &&
 // $U1_RESOURCE_PATH/u1b200_tunecache.tsv (the reference's tunecache.csv
 // location rule, src/tune.cpp:160-232).  U1_TUNE=0 disables tuning.
 namespace {
+struct TuneChoice {
+  int variant, threads;
+  bool duo;  // two phases per launch where the geometry allows (one-site kernel for the others)
+};
 struct TuneCache {
   std::mutex mu;
   bool loaded = false;
-  std::map<std::string, std::pair<int, int>> best;  // key -> (variant, threads per block)
+  std::map<std::string, TuneChoice> best;
 };
 TuneCache &tune_cache() {
   static TuneCache c;
@@ -1213,7 +1268,7 @@ void tune_load_locked(TuneCache &c) {
     if (line.empty() || line[0] == '#') continue;
     const size_t t1 = line.find('\t');
     if (t1 == std::string::npos) continue;
-    // key <tab> variant <tab> microseconds per sweep [<tab> threads per block]
+    // key <tab> variant <tab> microseconds per sweep [<tab> threads per block [<tab> two phases per launch]]
     std::vector<std::string> col;
     size_t a = 0;
     while (true) {
@@ -1225,14 +1280,15 @@ void tune_load_locked(TuneCache &c) {
     if (col.size() < 2) continue;
     const int v = std::atoi(col[1].c_str());
     const int threads = col.size() >= 4 ? std::atoi(col[3].c_str()) : 256;
-    if (v >= U1V_PAIR32 && v <= U1V_QUAD && block_valid(threads)) c.best[col[0]] = {v, threads};
+    const bool duo = col.size() >= 5 && std::atoi(col[4].c_str()) != 0;
+    if (v >= U1V_PAIR32 && v <= U1V_QUAD && block_valid(threads)) c.best[col[0]] = {v, threads, duo};
   }
 }
-void tune_save(const std::string &key, int v, double us, int threads) {
+void tune_save(const std::string &key, const TuneChoice &t, double us) {
   const std::string f = tune_file();
   if (f.empty()) return;
   std::ofstream out(f, std::ios::app);
-  if (out) out << key << '\t' << v << '\t' << us << '\t' << threads << '\n';
+  if (out) out << key << '\t' << t.variant << '\t' << us << '\t' << t.threads << '\t' << (t.duo ? 1 : 0) << '\n';
 }
 }  // namespace
 
@@ -1243,19 +1299,22 @@ static int tune_update(u1_lattice *lat, u1_rng *rng, bool use_cache) {
     std::lock_guard<std::mutex> lock(c.mu);
     tune_load_locked(c);
     auto it = c.best.find(key);
-    if (it != c.best.end() && variant_valid(lat, it->second.first)) {
-      lat->variant = it->second.first;
-      lat->block = it->second.second;
+    if (it != c.best.end() && variant_valid(lat, it->second.variant)) {
+      lat->variant = it->second.variant;
+      lat->block = it->second.threads;
+      lat->duo = it->second.duo;
       drop_graphs(lat);
       return U1_OK;
     }
   }
-  std::vector<std::pair<int, int>> cand;  // (variant, threads per block)
+  std::vector<TuneChoice> cand;
   for (int v : {U1V_PAIR32, U1V_QUAD, U1V_PAIR, U1V_SINGLE})  // the persistent sweep is opt-in (u1_wave.cuh)
     if (variant_valid(lat, v))
       for (int t : {256, 192, 128, 96, 64})
-        if (v != U1V_QUAD || t <= 128) cand.push_back({v, t});
-  std::pair<int, int> best = cand[0];
+        if (v != U1V_QUAD || t <= 128) cand.push_back({v, t, false});
+  if (duo_fits(lat))
+    for (int t : {256, 192, 128}) cand.push_back({U1V_SINGLE, t, true});
+  TuneChoice best = cand[0];
   double best_us = -1.0;
   if (cand.size() > 1) {
     const size_t n = (size_t)lat->g.V * lat->g.dims;
@@ -1278,8 +1337,9 @@ static int tune_update(u1_lattice *lat, u1_rng *rng, bool use_cache) {
     bool warmed = false;
     for (size_t ci : order) {
       const auto &vt = cand[ci];
-      lat->variant = vt.first;
-      lat->block = vt.second;
+      lat->variant = vt.variant;
+      lat->block = vt.threads;
+      lat->duo = vt.duo;
       cudaGraphExec_t ex = nullptr;
       rc = capture_graph(lat, [&]() { return issue_sweep(lat, lat->links, rng, 1, 4, 0, nullptr, true); }, &ex);
       double us = 0.0;
@@ -1298,8 +1358,8 @@ static int tune_update(u1_lattice *lat, u1_rng *rng, bool use_cache) {
       if (ex) cudaGraphExecDestroy(ex);
       if (rc) break;
       if (u1i::tune_verbose())
-        std::fprintf(stderr, "u1_tune %s: variant %d, %d threads: %.1f us per sweep\n", key.c_str(), vt.first,
-                     vt.second, us);
+        std::fprintf(stderr, "u1_tune %s: variant %d, %d threads%s: %.1f us per sweep\n", key.c_str(), vt.variant,
+                     vt.threads, vt.duo ? ", two phases per launch" : "", us);
       if (cand_us[ci] < 0.0 || us < cand_us[ci]) cand_us[ci] = us;
     }
     for (size_t k = 0; k < cand.size() && !rc; ++k)
@@ -1310,16 +1370,18 @@ static int tune_update(u1_lattice *lat, u1_rng *rng, bool use_cache) {
     if (rc) {
       lat->variant = U1V_AUTO;
       lat->block = 256;
+      lat->duo = false;
       return rc;
     }
   }
-  lat->variant = best.first;
-  lat->block = best.second;
+  lat->variant = best.variant;
+  lat->block = best.threads;
+  lat->duo = best.duo;
   drop_graphs(lat);
   std::lock_guard<std::mutex> lock(c.mu);
   tune_load_locked(c);
   c.best[key] = best;
-  tune_save(key, best.first, best_us, best.second);
+  tune_save(key, best, best_us);
   return U1_OK;
 }
 
@@ -1341,6 +1403,7 @@ extern "C" int u1_lattice_set_variant(u1_lattice *lat, int variant) {
     return fail(U1_ERR_INVALID, "u1_lattice_set_variant: variant not valid for this geometry (pair variants need Nx/2 even)");
   lat->variant = variant;
   lat->explicit_variant = variant != U1V_AUTO;
+  lat->duo = false;
   drop_graphs(lat);
   return U1_OK;
 }
@@ -1366,6 +1429,7 @@ extern "C" int u1_lattice_set_block(u1_lattice *lat, int threads) {
   if (!block_valid(threads))
     return fail(U1_ERR_INVALID, "u1_lattice_set_block: threads per block must be 32, 64, ..., 256");
   lat->block = threads;
+  lat->duo = false;  // an explicit block size is for one phase per launch
   drop_graphs(lat);
   return U1_OK;
 }

@@ -12,6 +12,16 @@
 #include "u1_geom.cuh"
 
 namespace u1b {
+// Layout of two phases in one launch (u1_duo.cuh).
+struct DuoK {
+  int rows;     // threads of a block that hold sites
+  int span;     // A = 2: consecutive sites (x0, x1) a block takes at each chain position
+  int len;      // A = 2: chain positions, lcm(N2, N3)
+  int groups;   // A = 2: blocks per chain class, N0/2 N1 / span
+  int blocks;
+  int threads;
+  FastDivK fspan, fgroups, fn2, fn3;
+};
 // Layout of a sweep in one thread-block cluster (u1_cluster.cuh).
 struct ClusterK {
   int blocks;   // blocks of the cluster
@@ -78,6 +88,7 @@ struct u1_lattice {
   int variant = U1V_AUTO;          // update kernel variant (U1V_AUTO: tune on first update)
   int block = 256;                 // threads per block of the phase kernels (tuned with the variant)
   bool explicit_variant = false;   // set by u1_lattice_set_variant (else chosen automatically)
+  bool duo = false;                // two phases per launch (u1_duo.cuh), chosen by the tuner with U1V_SINGLE
   int cluster_ok = -1;             // sweeps as one cluster launch: -1 unknown, 0 no, 1 yes (layout: cluster)
   u1b::ClusterK cluster{};
   int remap_block = -1;            // block size remap_sms was worked out for

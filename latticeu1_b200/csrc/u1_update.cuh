@@ -181,7 +181,9 @@ struct Chk {
 #endif
 };
 
-enum : int { CHK_READ = 0, CHK_OWN = 1, CHK_WRITE = 2 };  // another thread's link / the thread's own / a store
+// another thread's link / the thread's own / a store / a link that a thread of
+// the same block stores later in the launch, after a barrier (no race mark)
+enum : int { CHK_READ = 0, CHK_OWN = 1, CHK_WRITE = 2, CHK_LIVE = 3 };
 
 __device__ __forceinline__ Chk make_chk(const UpdArgs &a) {
 #ifdef U1_BOUNDS_CHECK
@@ -210,7 +212,7 @@ __device__ __forceinline__ bool chk(const Chk &c, const float2 *slab, int idx) {
     }
     return false;
   }
-  if (c.shadow != nullptr && KIND != CHK_OWN) {
+  if (c.shadow != nullptr && KIND != CHK_OWN && KIND != CHK_LIVE) {
     unsigned *m = c.shadow + ((slab + idx) - c.base);
 #pragma unroll
     for (int k = 0; k < W; ++k) {
@@ -233,6 +235,12 @@ __device__ __forceinline__ bool chk(const Chk &c, const float2 *slab, int idx) {
 __device__ __forceinline__ float2 ld1(const float2 *slab, int idx, const Chk &ck) {
   if (!chk<1, CHK_READ>(ck, slab, idx)) return make_float2(0.f, 0.f);
   return __ldg(slab + idx);
+}
+
+// One such link, through the coherent path.
+__device__ __forceinline__ float2 ld_live(const float2 *slab, int idx, const Chk &ck) {
+  if (!chk<1, CHK_LIVE>(ck, slab, idx)) return make_float2(0.f, 0.f);
+  return __ldca(slab + idx);
 }
 
 // Work item of block b of G in a phase with a.rev set: the last one first.

@@ -87,3 +87,58 @@ def test_cluster_sweep_in_multilevel(ctx, monkeypatch):
         lat.close()
     for r in res[1:]:
         assert np.array_equal(r[0], res[0][0]) and np.array_equal(r[1], res[0][1]) and r[2] == res[0][2]
+
+
+# planes and diagonals of one to several blocks, partly filled blocks, the largest
+# plane (512 sites), diagonals that are too long (22 x 18 x 14 x 30: only the planes
+# pair up), Nx/2 odd, extents of 2
+DUO = [(4, (8, 4, 6, 6)), (4, (4, 8, 2, 2)), (4, (16, 16, 16, 16)), (4, (6, 10, 12, 4)), (4, (22, 18, 14, 30)),
+       (4, (64, 16, 4, 6)), (4, (20, 20, 20, 20)), (4, (10, 12, 32, 16)), (3, (40, 18, 0, 22)), (3, (2, 4, 0, 6)),
+       (3, (34, 30, 0, 10))]
+
+
+def _duo_child(out):
+    """Every geometry with two phases per launch (as cached by the tuner) and with the one-site kernel."""
+    from latticeu1_b200 import Context, Lattice, Rng
+    ctx = Context(0)
+    res = {}
+    for k, (dims, N) in enumerate(DUO):
+        for window in (None, (0.7, 3)):
+            a = _chain(ctx, dims, N, 0.8, 0, window=window)
+            b = _chain(ctx, dims, N, 0.8, 3, window=window)
+            res[f"{k}_{window is None}"] = np.array([np.array_equal(a[0], b[0]), a[2] == b[2]])
+    ml = []
+    for variant in (0, 3):
+        lat = Lattice(ctx, 4, (16, 16, 16, 16), 0.95)
+        if variant:
+            lat.set_variant(variant)
+        rng = Rng(ctx, 3)
+        lat.hot_start(rng)
+        lat.update(rng, 1, 1)
+        ml.append((lat.multilevel(rng, 1, 1, 2, 1, 1, 2), lat.export_angles()))
+    res["multilevel"] = np.array([np.array_equal(ml[0][0], ml[1][0]), np.array_equal(ml[0][1], ml[1][1])])
+    np.savez(out, **res)
+
+
+def test_two_phases_per_launch(ctx, tmp_path):
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    import torch
+    name = torch.cuda.get_device_name(0)
+    lines = []
+    for k, (dims, N) in enumerate(DUO):
+        g = {3: (N[0], N[1], N[3], 1), 4: N}[dims]
+        lines.append(f"{name}|update|{dims}|{'x'.join(map(str, g))}\t3\t1.0\t{(128, 192, 256)[k % 3]}\t1\n")
+    (tmp_path / "u1b200_tunecache.tsv").write_text("".join(lines))
+    root = Path(__file__).resolve().parent.parent
+    env = dict(os.environ, U1_RESOURCE_PATH=str(tmp_path), U1_CLUSTER="0", PYTHONPATH=f"{root}:{root / 'tests'}")
+    env.pop("U1_TUNE", None)
+    out = tmp_path / "r.npz"
+    subprocess.run([sys.executable, "-c", f"import test_update_routes as t; t._duo_child({str(out)!r})"], env=env,
+                   check=True, timeout=300)
+    assert (tmp_path / "u1b200_tunecache.tsv").read_text() == "".join(lines)  # every geometry came from the cache
+    for k, v in np.load(out).items():
+        assert v.all(), (k, v)

@@ -23,6 +23,22 @@ from ._lib import check, lib, u1_geom
 __all__ = ["WilsonAction", "wilson_action", "topological_charge"]
 
 
+# The raw handle of a device's current stream: torch.cuda.current_stream builds a
+# Stream object for it, which costs more than the kernel launch behind it.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or \
+    (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
+def call_on_stream(device: torch.device, fn, name: str, *args) -> None:
+    """fn(*args, stream) with `device` current and its current stream."""
+    index = device.index
+    if torch.cuda.current_device() == index:
+        check(fn(*args, _raw_stream(index)), name)
+        return
+    with torch.cuda.device(device):
+        check(fn(*args, _raw_stream(index)), name)
+
+
 def make_geom(dims: int, N: Sequence[int], beta: float, aniso: float = 1.0) -> tuple[u1_geom, int]:
     """The ABI geometry and the link count V*dims (validated by the library)."""
     N = list(N) + [0] * (4 - len(N))
@@ -52,15 +68,16 @@ def _as_batch(theta: torch.Tensor, nlinks: int) -> torch.Tensor:
 def _forward_raw(g: u1_geom, theta: torch.Tensor) -> torch.Tensor:
     """(B, 2) float64: action and (2D) topological charge per configuration."""
     B = theta.shape[0]
-    nbytes = C.c_size_t()
-    check(lib.u1_action_workspace_bytes(C.byref(g), B, C.byref(nbytes)), "u1_action_workspace_bytes")
-    with torch.cuda.device(theta.device):
-        ws = torch.empty(max(1, nbytes.value // 8), dtype=torch.float64, device=theta.device)
-        out = torch.empty((B, 2), dtype=torch.float64, device=theta.device)
-        stream = torch.cuda.current_stream(theta.device).cuda_stream
-        check(lib.u1_wilson_action(C.byref(g), C.c_void_p(theta.data_ptr()), _dtype_code(theta), B,
-                                   C.c_void_p(ws.data_ptr()), C.c_void_p(out.data_ptr()), C.c_void_p(stream)),
-              "u1_wilson_action")
+    sizes = g.__dict__.setdefault("workspace", {})  # doubles of workspace by batch size
+    n = sizes.get(B)
+    if n is None:
+        nbytes = C.c_size_t()
+        check(lib.u1_action_workspace_bytes(C.byref(g), B, C.byref(nbytes)), "u1_action_workspace_bytes")
+        n = sizes[B] = max(1, nbytes.value // 8)
+    ws = torch.empty(n, dtype=torch.float64, device=theta.device)
+    out = torch.empty((B, 2), dtype=torch.float64, device=theta.device)
+    call_on_stream(theta.device, lib.u1_wilson_action, "u1_wilson_action", g, theta.data_ptr(), _dtype_code(theta), B,
+                   ws.data_ptr(), out.data_ptr())
     return out
 
 
@@ -75,14 +92,12 @@ class _WilsonActionFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_s: torch.Tensor):
         (theta,) = ctx.saved_tensors
-        scale = grad_s.detach().to(torch.float64).contiguous()
+        scale = grad_s.detach()
+        if scale.dtype != torch.float64 or not scale.is_contiguous():
+            scale = scale.to(torch.float64).contiguous()
         grad = torch.empty_like(theta)
-        with torch.cuda.device(theta.device):
-            stream = torch.cuda.current_stream(theta.device).cuda_stream
-            check(lib.u1_wilson_action_grad(C.byref(ctx.g), C.c_void_p(theta.data_ptr()), _dtype_code(theta),
-                                            theta.shape[0], C.c_void_p(scale.data_ptr()),
-                                            C.c_void_p(grad.data_ptr()), C.c_void_p(stream)),
-                  "u1_wilson_action_grad")
+        call_on_stream(theta.device, lib.u1_wilson_action_grad, "u1_wilson_action_grad", ctx.g, theta.data_ptr(),
+                       _dtype_code(theta), theta.shape[0], scale.data_ptr(), grad.data_ptr())
         return grad, None
 
 

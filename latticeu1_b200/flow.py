@@ -34,7 +34,7 @@ import torch
 from torch import nn
 
 from ._lib import check, lib
-from .action import WilsonAction
+from .action import WilsonAction, call_on_stream
 
 __all__ = ["Flow2D", "eo_permutation", "plaquettes_no", "independence_mh", "tau_int", "sample_mc",
            "plain_chain_q", "run_experiment"]
@@ -132,9 +132,8 @@ class _FusedLayer(torch.autograd.Function):
         ld = torch.empty(th.shape[0], device=th.device)
         fn, name = ((lib.u1_flow_layer_inverse, "u1_flow_layer_inverse") if inverse
                     else (lib.u1_flow_layer_forward, "u1_flow_layer_forward"))
-        with torch.cuda.device(th.device):
-            check(fn(_p(th), _p(out), _p(ld), th.shape[0], L, mu, off, K, H, _p(W1), _p(B1), _p(W2), _p(B2),
-                     C.c_float(slope), _stream(th)), name)
+        call_on_stream(th.device, fn, name, th.data_ptr(), out.data_ptr(), ld.data_ptr(), th.shape[0], L, mu, off, K,
+                       H, W1.data_ptr(), B1.data_ptr(), W2.data_ptr(), B2.data_ptr(), slope)
         ctx.save_for_backward(th, W1, B1, W2, B2)
         ctx.meta = meta
         ctx.inverse = inverse
@@ -154,9 +153,9 @@ class _FusedLayer(torch.autograd.Function):
         gth = torch.empty_like(th)
         part = torch.empty((B, nw), device=th.device)
         wg = torch.empty(nw, device=th.device)
-        with torch.cuda.device(th.device):
-            check(fn(_p(th), _p(g_out), _p(g_ld), _p(gth), _p(part), _p(wg), B, L, mu, off, K, H, _p(W1), _p(B1),
-                     _p(W2), _p(B2), C.c_float(slope), _stream(th)), name)
+        call_on_stream(th.device, fn, name, th.data_ptr(), g_out.data_ptr(), None if g_ld is None else g_ld.data_ptr(),
+                       gth.data_ptr(), part.data_ptr(), wg.data_ptr(), B, L, mu, off, K, H, W1.data_ptr(),
+                       B1.data_ptr(), W2.data_ptr(), B2.data_ptr(), slope)
         o = 0
         gW1 = wg[o:o + H * 18].view_as(W1)
         o += H * 18

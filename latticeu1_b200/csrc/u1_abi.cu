@@ -1111,11 +1111,18 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
   if (var == U1V_WAVE) return launch_wave(lat, links, rng, metrop, ovrn, meas_partials);
   const int D = lat->g.dims;
   const int total = 2 * D * (metrop + ovrn);
-  int phase = 0;
+  int phase = 0, launched = 0;
   // two phases per launch: an automatically tuned lattice whose tuner found it fastest
   DuoK duo[2];
+  QuadDuoK qduo;
+  SmOrder qorder{};
   bool pair_up[2] = {false, false};
-  if (lat->duo && src != SRC_REPLAY && D >= 3) {
+  const bool quads = var == U1V_QUAD;
+  if (lat->duo && src != SRC_REPLAY && quads) {
+    pair_up[0] = quad_duo_layout(lat->g, lat->block, lat->ctx->prop.multiProcessorCount, qduo);
+    // the SM-local order where both this grid and the four-site one run as one wave
+    if (pair_up[0]) qorder = sm_order(qduo.blocks, qduo.one_wave ? sms : 0);
+  } else if (lat->duo && src != SRC_REPLAY && D >= 3) {
     pair_up[0] = duo_layout(lat->g, 0, lat->block, duo[0]);
     pair_up[1] = D == 4 && duo_layout(lat->g, 2, lat->block, duo[1]);
   }
@@ -1125,8 +1132,16 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
     if ((a.mu & 1) == 0 && a.mu < 3 && pair_up[a.mu / 2] &&
         !(meas_partials && phase >= total - 2 * D && a.p == 1)) {  // not where the last pass measures
       phase += 2;
-      a.rev = 0;
-      int rc = launch_duo(D, a.mu, a, duo[a.mu / 2], lat->stream, met, src);
+      ++launched;
+      a.rev = (quads && alternate && (launched & 1) == 0) ? 1 : 0;
+      int rc;
+      if (quads) {
+        UpdArgs d = a;
+        d.order = qorder;
+        rc = launch_quad_duo(d, qduo, lat->stream, met, src);
+      } else {
+        rc = launch_duo(D, a.mu, a, duo[a.mu / 2], lat->stream, met, src);
+      }
       ++a.mu;
 #ifdef U1_BOUNDS_CHECK
       if (rc == U1_OK) rc = u1i::chk_phase_end(lat->stream, a.shadow, (size_t)D * lat->g.V, a.chk);
@@ -1134,7 +1149,8 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
       return rc;
     }
     ++phase;
-    a.rev = (alternate && (phase & 1) == 0) ? 1 : 0;  // every second phase runs its blocks backwards
+    ++launched;
+    a.rev = (alternate && (launched & 1) == 0) ? 1 : 0;  // every second launch runs its blocks backwards
     int rc;
     // the last pass is phases total-2D+1 .. total; its parity-1 half with mu >= 1 measures
     if (meas_partials && phase > total - 2 * D && a.p == 1 && a.mu >= 1)
@@ -1232,7 +1248,7 @@ static bool block_valid(int threads) { return threads >= 32 && threads <= 256 &&
 namespace {
 struct TuneChoice {
   int variant, threads;
-  bool duo;  // two phases per launch where the geometry allows (one-site kernel for the others)
+  bool duo;  // two phases per launch where the geometry allows (one- or four-site kernel, by the variant)
 };
 struct TuneCache {
   std::mutex mu;
@@ -1314,6 +1330,13 @@ static int tune_update(u1_lattice *lat, u1_rng *rng, bool use_cache) {
         if (v != U1V_QUAD || t <= 128) cand.push_back({v, t, false});
   if (duo_fits(lat))
     for (int t : {256, 192, 128}) cand.push_back({U1V_SINGLE, t, true});
+  int last_rows = 0;
+  for (int t : {256, 192, 128}) {  // block sizes that hold the same planes are one candidate
+    QuadDuoK d;
+    if (!quad_duo_layout(lat->g, t, lat->ctx->prop.multiProcessorCount, d) || d.rows == last_rows) continue;
+    last_rows = d.rows;
+    cand.push_back({U1V_QUAD, t, true});
+  }
   TuneChoice best = cand[0];
   double best_us = -1.0;
   if (cand.size() > 1) {

@@ -22,6 +22,18 @@ struct DuoK {
   int threads;
   FastDivK fspan, fgroups, fn2, fn3;
 };
+// The same for directions 0 and 1 with four sites per thread (u1_quad_duo.cu).
+struct QuadDuoK {
+  int rows;  // threads of a block that hold sites: whole (x0, x1)-planes
+  int threads;
+  int blocks;
+  int regs;  // register bound of the kernel: 96, 72 or 64
+  bool one_wave;
+};
+// Blocks of about `target` threads; false where the lattice has no such layout.
+bool quad_duo_layout(const GeomK &g, int target, int sms, QuadDuoK &d);
+struct UpdArgs;
+int launch_quad_duo(const UpdArgs &a, const QuadDuoK &d, cudaStream_t s, bool met, int src);
 // Layout of a sweep in one thread-block cluster (u1_cluster.cuh).
 struct ClusterK {
   int blocks;   // blocks of the cluster
@@ -88,7 +100,7 @@ struct u1_lattice {
   int variant = U1V_AUTO;          // update kernel variant (U1V_AUTO: tune on first update)
   int block = 256;                 // threads per block of the phase kernels (tuned with the variant)
   bool explicit_variant = false;   // set by u1_lattice_set_variant (else chosen automatically)
-  bool duo = false;                // two phases per launch (u1_duo.cuh), chosen by the tuner with U1V_SINGLE
+  bool duo = false;                // two phases per launch, chosen by the tuner with U1V_SINGLE (u1_duo.cuh) or U1V_QUAD (u1_quad_duo.cu)
   int cluster_ok = -1;             // sweeps as one cluster launch: -1 unknown, 0 no, 1 yes (layout: cluster)
   u1b::ClusterK cluster{};
   int remap_block = -1;            // block size remap_sms was worked out for

@@ -596,10 +596,12 @@ __device__ __forceinline__ Quad2 ld_quad(const float2 *base, int idx, const Chk 
                : "memory");
   return q;
 }
-// The same through the coherent path (the thread's own links, stored later).
+// The same through the coherent path: the thread's own links, stored later
+// (CHK_OWN), or links that this launch stores after a barrier (CHK_LIVE).
+template <int KIND = CHK_OWN>
 __device__ __forceinline__ Quad2 ld_quad_own(const float2 *slab, int idx, const Chk &ck) {
   Quad2 q;
-  if (!chk<4, CHK_OWN>(ck, slab, idx)) {
+  if (!chk<4, KIND>(ck, slab, idx)) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) q.s[s] = make_float2(0.f, 0.f);
     return q;
@@ -645,17 +647,19 @@ __device__ __forceinline__ Row4 row4(const GeomK &g, int x0, int k) {
   return r;
 }
 // The link of the neighbouring quad: `mine` is what this lane's quad lends.
+template <bool LIVE = false>
 __device__ __forceinline__ float2 row4_edge(const float2 *base, int idx, const Row4 &r, float2 mine, bool used,
                                             const Chk &ck) {
   float2 v = make_float2(__shfl_sync(r.mask, mine.x, r.src & 31), __shfl_sync(r.mask, mine.y, r.src & 31));
   if (r.any)
-    if (r.out && used) v = ld1(base, idx + r.edge, ck);
+    if (r.out && used) v = LIVE ? ld_live(base, idx + r.edge, ck) : ld1(base, idx + r.edge, ck);
   return v;
 }
 // Links at x + e0 of the sites of quad idx.
+template <bool LIVE = false>
 __device__ __forceinline__ Quad2 ld_quad_fwd0(const float2 *base, int idx, const Row4 &r, const Chk &ck) {
-  Quad2 q = ld_quad(base, idx, ck);
-  const float2 v = row4_edge(base, idx, r, q.s[0], r.odd, ck);
+  Quad2 q = LIVE ? ld_quad_own<CHK_LIVE>(base, idx, ck) : ld_quad(base, idx, ck);
+  const float2 v = row4_edge<LIVE>(base, idx, r, q.s[0], r.odd, ck);
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
     const float2 n = s < 3 ? q.s[s < 3 ? s + 1 : 3] : v;
@@ -686,52 +690,43 @@ __device__ __forceinline__ void ld_row5(const float2 *base, int idx, const Row4 
   }
 }
 
-// Body of the four-sites-per-thread update for EO sites i..i+3 (i a multiple
-// of 4) of the phase (a.p, MU); every site's staple and update use the same
-// operations in the same order as the other bodies (bit-identical links).
-// MEAS: also add the plaquettes (nu < MU, MU) of the four sites from their
-// staple terms into *meas (as update_pair_body).
-template <int D, int MU, bool MET, int SRC, bool MEAS = false>
-__device__ __forceinline__ void update_quad_body(const UpdArgs a, int i, float2 *meas = nullptr) {
-  // site decode and neighbour steps (pure arithmetic) before the wait for
-  // the previous phase, overlapping its tail
-  int x[4], k;
-  eo_decode_fast<D>(a.g, i, a.p, x, k);
-  int fwd[4], bwd[4];
-  eo_steps<D>(a.g, x, k, fwd, bwd);  // steps of site i; sites i+1..i+3 share those along x1..x3
-  Row4 row = row4(a.g, x[0], k);
-  // freeze rule, src/multilevel.cu:41 (rows lie in one time slice: they are updated or not as a whole)
-  const bool active = i < a.g.Vh && (MEAS || MU == 3 || a.ml == 0 || (x[D - 1] & (a.ml - 1)) != 0);
-  row.mask = __ballot_sync(0xffffffffu, active);
-  row.any = __any_sync(0xffffffffu, row.out);
-  phase_entry<MET>(a);
-  if (!active) return;
+// Staple terms of the links in direction MU of the four sites i..i+3; mA, mD:
+// measurement sums (MEAS), see update_single_body.
+struct QuadSums {
+  float2 ss[4], st[4], mA[4], mD[4];
+};
+// GIVEN: a direction whose parity-p links at x and at x + e_MU - e_GIVEN the
+// caller holds (C0, D0) instead of loading them; LIVE: one whose parity-p links
+// this launch stores later (both: u1_quad_duo.cu, else -1).
+template <int D, int MU, bool MEAS, int GIVEN = -1, int LIVE = -1>
+__device__ __forceinline__ QuadSums quad_staples(const UpdArgs &a, int i, const int fwd[4], const int bwd[4],
+                                                 const Row4 &row, const Chk &ck, const Quad2 &C0 = Quad2{},
+                                                 const Quad2 &D0 = Quad2{}) {
   const int q = 1 - a.p;
   const int V = a.g.V, Vh = a.g.Vh;
   const float2 *lat = a.lat;
   const float2 *Lq_mu = lat + MU * V + q * Vh;
-  const Chk ck = make_chk(a);
-  float2 ss[4], st[4], mA[4], mD[4];  // mA, mD: measurement sums (MEAS), see update_single_body
+  QuadSums o;
   // the first term of each sum is stored, not added to 0 (equal up to the sign of a zero)
   constexpr int kFirst = MU == 0 ? 1 : 0;
 #pragma unroll
-  for (int s = 0; s < 4; ++s) ss[s] = st[s] = mA[s] = mD[s] = make_float2(0.f, 0.f);
+  for (int s = 0; s < 4; ++s) o.ss[s] = o.st[s] = o.mA[s] = o.mD[s] = make_float2(0.f, 0.f);
 #pragma unroll
   for (int nu = 0; nu < D; ++nu) {
     if (nu == MU) continue;
     const float2 *Lp_nu = lat + nu * V + a.p * Vh;
     const float2 *Lq_nu = lat + nu * V + q * Vh;
     Quad2 A, B, C, Dd, E, F;
-    C = ld_quad(Lp_nu, i, ck);
+    C = nu == GIVEN ? C0 : nu == LIVE ? ld_quad_own<CHK_LIVE>(Lp_nu, i, ck) : ld_quad(Lp_nu, i, ck);
     if (MU == 0) {  // nu != 0: steps along nu shared, along x0 per site
       A = ld_quad_fwd0(Lq_nu, i, row, ck);
       B = ld_quad(Lq_mu, i + fwd[nu], ck);
-      Dd = ld_quad_fwd0(Lp_nu, i + bwd[nu], row, ck);
+      Dd = nu == LIVE ? ld_quad_fwd0<true>(Lp_nu, i + bwd[nu], row, ck) : ld_quad_fwd0(Lp_nu, i + bwd[nu], row, ck);
       E = ld_quad(Lq_mu, i + bwd[nu], ck);
       F = ld_quad(Lq_nu, i + bwd[nu], ck);
     } else if (nu == 0) {  // MU != 0
       A = ld_quad(Lq_nu, i + fwd[MU], ck);
-      Dd = ld_quad_bwd0(Lp_nu, i + fwd[MU], row, ck);
+      Dd = nu == GIVEN ? D0 : ld_quad_bwd0(Lp_nu, i + fwd[MU], row, ck);
       F = ld_quad_bwd0(Lq_nu, i, row, ck);
       float2 w[5];
       ld_row5(Lq_mu, i, row, w, ck);
@@ -752,37 +747,68 @@ __device__ __forceinline__ void update_quad_body(const UpdArgs a, int i, float2 
       const float2 up = cmulc(cmulc(A.s[s], B.s[s]), C.s[s]), lo = cmul(cconjmul(Dd.s[s], E.s[s]), F.s[s]);
       const float2 t = cadd(up, lo);
       if (MU == D - 1 || nu == D - 1)
-        st[s] = (MU == D - 1 ? nu == kFirst : true) ? t : cadd(st[s], t);
+        o.st[s] = (MU == D - 1 ? nu == kFirst : true) ? t : cadd(o.st[s], t);
       else
-        ss[s] = nu == kFirst ? t : cadd(ss[s], t);
+        o.ss[s] = nu == kFirst ? t : cadd(o.ss[s], t);
       if (MEAS && nu < MU) {
-        if (MU != D - 1) mA[s] = cadd(mA[s], t);  // for MU = D-1 every nu < MU term is in st
-        mD[s] = cadd(mD[s], csub(up, lo));
+        if (MU != D - 1) o.mA[s] = cadd(o.mA[s], t);  // for MU = D-1 every nu < MU term is in st
+        o.mD[s] = cadd(o.mD[s], csub(up, lo));
       }
     }
   }
-  float2 *own_slab = a.lat + MU * V + a.p * Vh;
+  return o;
+}
+
+// The new links N of the four sites from their staple terms, stored.
+template <int D, int MU, bool MET, int SRC>
+__device__ __forceinline__ void quad_links(const UpdArgs &a, int i, const QuadSums &o, const Chk &ck, float2 (&N)[4]) {
+  float2 *own_slab = a.lat + MU * a.g.V + a.p * a.g.Vh;
   const Quad2 U = ld_quad_own(own_slab, i, ck);
   // sites i, i+1 and i+2, i+3 share one Philox block each
   Philox4 blk0, blk1;
   if (MET && SRC != SRC_REPLAY) {
     const unsigned long long pass = *a.pass_dev + (unsigned long long)a.hit;
-    blk0 = u1_metropolis_block((uint32_t)(a.p * Vh + i), MU, a.chain, pass, a.key0, a.key1);
-    blk1 = u1_metropolis_block((uint32_t)(a.p * Vh + i + 2), MU, a.chain, pass, a.key0, a.key1);
+    blk0 = u1_metropolis_block((uint32_t)(a.p * a.g.Vh + i), MU, a.chain, pass, a.key0, a.key1);
+    blk1 = u1_metropolis_block((uint32_t)(a.p * a.g.Vh + i + 2), MU, a.chain, pass, a.key0, a.key1);
   }
-  float2 N[4];
 #pragma unroll
   for (int s = 0; s < 4; ++s)
-    N[s] = update_one<D, MU, MET, SRC>(a, i + s, cweigh(ss[s], a.c.w_ss, st[s], a.c.w_st), U.s[s],
+    N[s] = update_one<D, MU, MET, SRC>(a, i + s, cweigh(o.ss[s], a.c.w_ss, o.st[s], a.c.w_st), U.s[s],
                                        s < 2 ? &blk0 : &blk1);
   st_quad(own_slab, i, N, ck);
+}
+
+// Body of the four-sites-per-thread update for EO sites i..i+3 (i a multiple
+// of 4) of the phase (a.p, MU); every site's staple and update use the same
+// operations in the same order as the other bodies (bit-identical links).
+// MEAS: also add the plaquettes (nu < MU, MU) of the four sites from their
+// staple terms into *meas (as update_pair_body).
+template <int D, int MU, bool MET, int SRC, bool MEAS = false>
+__device__ __forceinline__ void update_quad_body(const UpdArgs a, int i, float2 *meas = nullptr) {
+  // site decode and neighbour steps (pure arithmetic) before the wait for
+  // the previous phase, overlapping its tail
+  int x[4], k;
+  eo_decode_fast<D>(a.g, i, a.p, x, k);
+  int fwd[4], bwd[4];
+  eo_steps<D>(a.g, x, k, fwd, bwd);  // steps of site i; sites i+1..i+3 share those along x1..x3
+  Row4 row = row4(a.g, x[0], k);
+  // freeze rule, src/multilevel.cu:41 (rows lie in one time slice: they are updated or not as a whole)
+  const bool active = i < a.g.Vh && (MEAS || MU == 3 || a.ml == 0 || (x[D - 1] & (a.ml - 1)) != 0);
+  row.mask = __ballot_sync(0xffffffffu, active);
+  row.any = __any_sync(0xffffffffu, row.out);
+  phase_entry<MET>(a);
+  if (!active) return;
+  const Chk ck = make_chk(a);
+  const QuadSums o = quad_staples<D, MU, MEAS>(a, i, fwd, bwd, row, ck);
+  float2 N[4];
+  quad_links<D, MU, MET, SRC>(a, i, o, ck, N);
   pdl_release_dependents();
   if (MEAS) {
     float re = 8.f * MU, im = 0.f;
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
-      re -= cre_mul((MU == D - 1) ? st[s] : mA[s], N[s]);
-      im += cim_mul(mD[s], N[s]);
+      re -= cre_mul((MU == D - 1) ? o.st[s] : o.mA[s], N[s]);
+      im += cim_mul(o.mD[s], N[s]);
     }
     *meas = make_float2(re, im);
   }

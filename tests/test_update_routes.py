@@ -97,12 +97,21 @@ DUO = [(4, (8, 4, 6, 6)), (4, (4, 8, 2, 2)), (4, (16, 16, 16, 16)), (4, (6, 10, 
        (3, (34, 30, 0, 10))]
 
 
-def _duo_child(out):
+# four sites per thread: rows of one to sixteen quads, rows that cross warps (24, 40),
+# extents of 2, partly filled blocks, planes of up to 1024 threads; register bounds 96
+# (few blocks), 72 (64 x 64 x 4 x 2; several waves of 288 threads) and 64 (planes above
+# 896 threads; several waves of 512, links above half the L2)
+QUAD_DUO = [(4, (8, 2, 2, 2)), (4, (8, 4, 4, 6)), (4, (16, 16, 16, 16)), (4, (24, 24, 4, 6)), (4, (40, 40, 4, 4)),
+            (4, (64, 64, 4, 2)), (4, (128, 64, 4, 4)), (4, (8, 4, 34, 34)), (4, (48, 48, 24, 20)),
+            (4, (64, 64, 24, 24)), (3, (16, 10, 0, 6)), (3, (32, 34, 0, 38))]
+
+
+def _duo_child(out, geometries=None):
     """Every geometry with two phases per launch (as cached by the tuner) and with the one-site kernel."""
     from latticeu1_b200 import Context, Lattice, Rng
     ctx = Context(0)
     res = {}
-    for k, (dims, N) in enumerate(DUO):
+    for k, (dims, N) in enumerate(geometries or DUO):
         for window in (None, (0.7, 3)):
             a = _chain(ctx, dims, N, 0.8, 0, window=window)
             b = _chain(ctx, dims, N, 0.8, 3, window=window)
@@ -120,7 +129,8 @@ def _duo_child(out):
     np.savez(out, **res)
 
 
-def test_two_phases_per_launch(ctx, tmp_path):
+@pytest.mark.parametrize("variant,geometries", [(3, "DUO"), (5, "QUAD_DUO")])
+def test_two_phases_per_launch(ctx, tmp_path, variant, geometries):
     import os
     import subprocess
     import sys
@@ -129,16 +139,16 @@ def test_two_phases_per_launch(ctx, tmp_path):
     import torch
     name = torch.cuda.get_device_name(0)
     lines = []
-    for k, (dims, N) in enumerate(DUO):
+    for k, (dims, N) in enumerate(globals()[geometries]):
         g = {3: (N[0], N[1], N[3], 1), 4: N}[dims]
-        lines.append(f"{name}|update|{dims}|{'x'.join(map(str, g))}\t3\t1.0\t{(128, 192, 256)[k % 3]}\t1\n")
+        lines.append(f"{name}|update|{dims}|{'x'.join(map(str, g))}\t{variant}\t1.0\t{(128, 192, 256)[k % 3]}\t1\n")
     (tmp_path / "u1b200_tunecache.tsv").write_text("".join(lines))
     root = Path(__file__).resolve().parent.parent
     env = dict(os.environ, U1_RESOURCE_PATH=str(tmp_path), U1_CLUSTER="0", PYTHONPATH=f"{root}:{root / 'tests'}")
     env.pop("U1_TUNE", None)
     out = tmp_path / "r.npz"
-    subprocess.run([sys.executable, "-c", f"import test_update_routes as t; t._duo_child({str(out)!r})"], env=env,
-                   check=True, timeout=300)
+    code = f"import test_update_routes as t; t._duo_child({str(out)!r}, t.{geometries})"
+    subprocess.run([sys.executable, "-c", code], env=env, check=True, timeout=300)
     assert (tmp_path / "u1b200_tunecache.tsv").read_text() == "".join(lines)  # every geometry came from the cache
     for k, v in np.load(out).items():
         assert v.all(), (k, v)

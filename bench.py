@@ -170,7 +170,7 @@ def ncu_batch_traffic_per_link_sweep(group_mb: int, lanes: int) -> tuple[float |
 
 # Sources the update kernels compile from: a committed ncu figure counts only
 # while their digest matches the one recorded beside it.
-UPDATE_KERNEL_SOURCES = ("u1_update.cuh", "u1_geom.cuh", "u1_cplx.cuh", "u1_philox.h")
+UPDATE_KERNEL_SOURCES = ("u1_update.cuh", "u1_quad_duo.cu", "u1_geom.cuh", "u1_cplx.cuh", "u1_philox.h")
 
 
 def update_kernel_digest() -> str:
@@ -541,7 +541,8 @@ def run_ours(args) -> None:
             "config": workload_config(N, beta, aniso, args.delta, args.nhits),
             "roofline": {"bound": "hbm",
                          "kernel": KERNEL_OF_VARIANT.get(lat.variant, "k_update") +
-                                   " (one (parity,mu) phase; step average)",
+                                   " (one (parity,mu) phase; step average over the phases, of which one launch "
+                                   "may run two)",
                          "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "traffic_source": traffic_note,
                          "dram_frac": (traffic / alg_bytes) if traffic else None,

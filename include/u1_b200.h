@@ -103,8 +103,11 @@ int u1_lattice_set_coupling(u1_lattice *lat, double beta, double aniso);
 int u1_lattice_set_graphs(u1_lattice *lat, int enable);
 /* Update kernel variants, all giving bit-identical links: 1 = two sites per
  * thread (32-register cap, 8 CTAs/SM), 2 = two sites per thread (no cap),
- * 3 = one site per thread, 5 = four sites per thread (72-register cap,
- * 256-bit loads, at most 128 threads per block: larger settings run 128); 0 = auto (tuned at the first u1_update among 1, 2, 3, 5).
+ * 3 = one site per thread, 5 = four sites per thread (72- or 80-register cap,
+ * 256-bit loads, at most 128 threads per block: larger settings run 128); 0 = auto: a
+ * lattice that fits one thread-block cluster runs whole sweeps as one launch
+ * (U1_CLUSTER=0 in the environment: never), any other is tuned at the first
+ * u1_update among 1, 2, 3, 5, and 3 and 5 also with two phases per launch.
  * The two-site variants need Nx/2 even, the four-site one Nx/2 a multiple
  * of 4.  4 = the whole sweep as one
  * persistent cooperative kernel with neighbour-local phase synchronisation
@@ -134,9 +137,10 @@ int u1_lattice_set_wave_wait(u1_lattice *lat, unsigned spin_limit, int stall_til
 int u1_lattice_set_metropolis(u1_lattice *lat, double delta, int nhits);
 int u1_lattice_get_metropolis(const u1_lattice *lat, double *delta, int *nhits);
 /* Replaces the reference's autotuner (tuneLaunch, src/tune.cpp:306-416):
- * times every valid variant (1, 2, 3, 5) at 64, 96, 128, 192 and 256 threads per block (5: up to 128) on a
- * few sweeps of this lattice from a backed-up state (links and rng pass
- * restored afterwards), keeps the fastest pair and caches it per (device,
+ * times every valid variant (1, 2, 3, 5) at 64, 96, 128, 192 and 256 threads per block (5: up to 128),
+ * and 3 and 5 with two phases per launch where the extents allow, on a few
+ * sweeps of this lattice from a backed-up state (links and rng pass restored
+ * afterwards), keeps the fastest choice and caches it per (device,
  * geometry); with U1_RESOURCE_PATH set the cache persists in
  * $U1_RESOURCE_PATH/u1b200_tunecache.tsv.  U1_TUNE=0 in the environment
  * turns the automatic first-update tuning off.  *variant gets the variant;
@@ -437,14 +441,15 @@ int u1_flow_layer_backward(const float *theta_in, const float *grad_theta_out, c
 /* The inverse coupling layer (no counterpart in the reference), arguments as
  * u1_flow_layer_forward: the same context net (the context plaquettes hold no
  * updated link, so the layer and its inverse see the same parameters), then
- * the inverse mixture transform of each active plaquette by bisection, the
+ * the inverse mixture transform of each active plaquette (bracketed Newton
+ * steps to the float resolution), the
  * link change that undoes a forward step, and logdet[b] = sum of log H' at the
  * solutions (the forward layer's log-det at the returned configuration). */
 int u1_flow_layer_inverse(const float *theta_in, float *theta_out, float *logdet, int batch, int L, int mu, int off,
                           int K, int hidden, const float *W1, const float *B1, const float *W2, const float *B2,
                           float slope, void *stream);
 /* Backward of u1_flow_layer_inverse (implicit differentiation at the
- * bisection solution), arguments as u1_flow_layer_backward. */
+ * solution), arguments as u1_flow_layer_backward. */
 int u1_flow_layer_inverse_backward(const float *theta_in, const float *grad_theta_out, const float *grad_logdet,
                                    float *grad_theta_in, float *wgrad_partials, float *wgrad, int batch, int L,
                                    int mu, int off, int K, int hidden, const float *W1, const float *B1,

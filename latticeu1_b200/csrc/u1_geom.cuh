@@ -84,16 +84,6 @@ struct CoupK {
   float w_st;  // xi    for plaquettes with a temporal link
 };
 
-__device__ __forceinline__ void eo_decode(const GeomK &g, int i, int p, int x[4]) {
-  int k = i % g.hN0;
-  int r = i / g.hN0;
-  x[1] = r % g.N[1];
-  r /= g.N[1];
-  x[2] = r % g.N[2];
-  x[3] = r / g.N[2];
-  x[0] = 2 * k + ((x[1] + x[2] + x[3] + p) & 1);
-}
-
 // Site of EO index i (parity p) via the fast divisors; k = i mod hN0.
 template <int D>
 __device__ __forceinline__ void eo_decode_fast(const GeomK &g, int i, int p, int x[4], int &k) {
@@ -141,8 +131,5 @@ __device__ __forceinline__ void eo_steps(const GeomK &g, const int x[4], int k, 
 __device__ __forceinline__ int eo_index(const GeomK &g, const int x[4]) {
   return (x[0] >> 1) + x[1] * g.es[1] + x[2] * g.es[2] + x[3] * g.es[3];
 }
-
-__device__ __forceinline__ int wrap_inc(int v, int n) { return (v + 1 == n) ? 0 : v + 1; }
-__device__ __forceinline__ int wrap_dec(int v, int n) { return (v == 0) ? n - 1 : v - 1; }
 
 }  // namespace u1b

@@ -111,16 +111,6 @@ __device__ __forceinline__ void finish_block_totals(double tot, double *smem, do
   if (threadIdx.x == 0) *counter = 0u;
 }
 
-// Store this block's NV totals, take a ticket; the last block sums all
-// partials in block order and writes out[k] = scale[k] * total_k.
-template <int NV>
-__device__ __forceinline__ void partials_finish(double (&v)[NV], double *smem, double *partials,
-                                                unsigned int *counter, double *out,
-                                                const double (&scale)[NV]) {
-  block_sum<NV>(v, smem);
-  finish_block_totals<NV>(v[0], smem, partials, counter, out, scale);
-}
-
 // Launch layout of the plaquette + Polyakov measurement.
 //  * blocks [0, nb_plaq): plaquettes.  pair != 0 (N0/2 even): thread t
 //    takes EO sites i = 2t, 2t+1 of both parities, whose neighbours along

@@ -3,12 +3,14 @@
 // The second phase needs of the first only the new links U_0(x) and
 // U_0(x + e1 - e0) (u1_duo.cuh), which lie in x's (x0, x1)-plane.  A block owns
 // whole planes, keeps the new U_0 in shared memory and runs both phases with a
-// block barrier between them: one launch boundary less in four phases, and of the
-// second phase's 20 quad loads three become shared-memory reads (C and D of the
-// plane (0, 1) and its row edges).  A phase of a large lattice is bound by those
-// loads (L1 wavefronts in cache, DRAM beyond it), one that fits the L2 by the
-// launch boundary as well.  Unlike u1_duo.cuh the loads of the second phase are
-// not issued before the first: 40 quad loads a thread do not fit the registers.
+// block barrier between them: one launch boundary less in four phases, and two of
+// the second phase's 17 quad loads (U_0 at x and at x + e1 - e0, with the row edge
+// of the latter) become shared-memory reads.  A phase of a large lattice is bound
+// by those loads (L1 wavefronts in cache, DRAM beyond it), one that fits the L2 by
+// the launch boundary as well.  Unlike u1_duo.cuh the loads of the second phase
+// are not issued before the first: 35 quad loads a thread do not fit the
+// registers.  In a batch, whose second lane already covers the boundaries, the
+// same made no difference (7.6 ms a sweep of 512 chains with and without).
 //
 // The register bound decides how many threads an SM holds, so there are three:
 // 96 registers where the grid is then still one wave, 72 where that makes it one

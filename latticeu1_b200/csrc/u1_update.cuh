@@ -30,52 +30,6 @@ __device__ __forceinline__ float2 ldg2(const float2 *p) { return __ldg(p); }
 __device__ __forceinline__ void pdl_wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release_dependents() { asm volatile("griddepcontrol.launch_dependents;" :::); }
 
-// Staple S of link (x, mu), x of parity p with EO index i_self, so that the
-// local action of the link is beta * Re(S * U_mu(x)).
-template <int D>
-__device__ __forceinline__ float2 staple_at(const float2 *__restrict__ lat, const GeomK &g,
-                                            const CoupK &c, const int x[4], int i_self, int p,
-                                            int mu) {
-  const int q = 1 - p;
-  const size_t offP = (size_t)p * g.Vh, offQ = (size_t)q * g.Vh;
-  const size_t Vmu = (size_t)mu * g.V;
-  int xm[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) xm[k] = (k == mu) ? wrap_inc(x[k], g.N[k]) : x[k];
-  const int i_xm = eo_index(g, xm);  // x + mu, parity q
-  float2 ss = make_float2(0.f, 0.f), st = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int nu = 0; nu < D; ++nu) {
-    if (nu == mu) continue;
-    const size_t Vnu = (size_t)nu * g.V;
-    int xn[4], xd[4], xmd[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      xn[k] = (k == nu) ? wrap_inc(x[k], g.N[k]) : x[k];
-      xd[k] = (k == nu) ? wrap_dec(x[k], g.N[k]) : x[k];
-      xmd[k] = (k == nu) ? wrap_dec(xm[k], g.N[k]) : xm[k];
-    }
-    const int i_xn = eo_index(g, xn);    // x + nu       parity q
-    const int i_xd = eo_index(g, xd);    // x - nu       parity q
-    const int i_xmd = eo_index(g, xmd);  // x + mu - nu  parity p
-    // upper: U_nu(x+mu) conj(U_mu(x+nu)) conj(U_nu(x))
-    float2 a = ldg2(lat + Vnu + offQ + i_xm);
-    float2 b = ldg2(lat + Vmu + offQ + i_xn);
-    float2 cc = ldg2(lat + Vnu + offP + i_self);
-    float2 up = cmulc(cmulc(a, b), cc);
-    // lower: conj(U_nu(x+mu-nu)) conj(U_mu(x-nu)) U_nu(x-nu)
-    float2 d = ldg2(lat + Vnu + offP + i_xmd);
-    float2 e = ldg2(lat + Vmu + offQ + i_xd);
-    float2 f = ldg2(lat + Vnu + offQ + i_xd);
-    float2 lo = cmul(cconjmul(d, e), f);
-    if (mu == g.tdir || nu == g.tdir)
-      st = cadd(st, cadd(up, lo));
-    else
-      ss = cadd(ss, cadd(up, lo));
-  }
-  return cweigh(ss, c.w_ss, st, c.w_st);
-}
-
 // 1/sqrt(v) of a v near 1: rsqrtf without its treatment of subnormal arguments.
 __device__ __forceinline__ float rsqrt_unit(float v) {
   float r;
@@ -158,7 +112,7 @@ struct UpdArgs {
 // the kernel never touches memory outside its half of the lattice.  With a
 // shadow array (one word per link of the buffer) every access is also marked:
 // bit 0 for a read of a link the thread does not own, +2 for a write.
-// k_chk_phase_end runs after every phase: a link written and also read by
+// k_chk_phase_end runs after every launch: a link written and also read by
 // another thread, or written twice, within one phase is a checkerboard race;
 // it counts them and clears the marks.  In the normal build Chk is empty and
 // every check folds to `true`.

@@ -19,10 +19,10 @@ even/odd layout.
 
 Library kernels on this path: the circular coupling transform and its
 inverse with analytic backward passes (u1_ncp_*), the Wilson action and its
-adjoint (u1_wilson_action*), and for proposals one fused kernel per coupling
-layer (u1_flow_layer_forward: context net, transform, link update, log-det).
-In training the 3x3 convolutions run through cuDNN in bfloat16 with FP32
-accumulation.
+adjoint (u1_wilson_action*), and, for proposals and for training at L <= 32,
+one fused kernel per coupling layer and direction (u1_flow_layer_*: context
+net, transform, link update, log-det).  Beyond that size the 3x3 convolutions
+of training run through cuDNN in bfloat16 with FP32 accumulation.
 """
 from __future__ import annotations
 

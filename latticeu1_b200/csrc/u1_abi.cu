@@ -1331,7 +1331,7 @@ static int tune_update(u1_lattice *lat, u1_rng *rng, bool use_cache) {
   if (duo_fits(lat))
     for (int t : {256, 192, 128}) cand.push_back({U1V_SINGLE, t, true});
   int last_rows = 0;
-  for (int t : {256, 192, 128}) {  // block sizes that hold the same planes are one candidate
+  for (int t : {256, 224, 192, 128}) {  // block sizes that hold the same planes are one candidate
     QuadDuoK d;
     if (!quad_duo_layout(lat->g, t, lat->ctx->prop.multiProcessorCount, d) || d.rows == last_rows) continue;
     last_rows = d.rows;

@@ -17,10 +17,10 @@
 // or holds as many threads as 64 do, 64 elsewhere (a plane of 512 threads at
 // 64^4: two blocks an SM instead of one).  Mean over the four phases of a
 // half-pass, us, overrelaxation, one phase a launch / this (B200): 24^3 x 32
-// (216 threads, 96 registers) 3.28 / 3.04, 24^3 x 48 (144, 72) 4.18 / 3.98, 32^4
-// (128, 72) 5.27 / 4.95, 48^4 (288, 72) 27.7 / 27.5 (Metropolis 34.2 / 31.9), 64^4
-// (512, 64) 101.0 / 95.7.  40^4 (224 threads of which 200 hold sites) is slower,
-// 12.9 / 13.1: the tuner chooses by timing.
+// (216 threads, 96 registers) 3.28 / 3.04, 24^3 x 48 (288, 96) 4.18 / 3.73
+// (a whole sweep 162 -> 152 us), 32^4 (128, 72) 5.27 / 4.95, 48^4 (288, 72) 27.7 /
+// 27.5 (Metropolis 34.2 / 31.9), 64^4 (512, 64) 101.0 / 95.7.  40^4 (224 threads of
+// which 200 hold sites) is slower, 12.9 / 13.1: the tuner chooses by timing.
 #include "u1_internal.h"
 #include "u1_update.cuh"
 
@@ -131,6 +131,7 @@ bool quad_duo_layout(const GeomK &g, int target, int sms, QuadDuoK &d) {
   if (g.dims < 3 || (g.hN0 & 3) != 0) return false;
   const long long plane = (long long)(g.hN0 / 4) * g.N[1];
   if (plane > 1024) return false;
+  if (target >= 256) target = 288;  // the largest block of the kernel with 96 registers
   const int planes = (int)(g.Vh / 4 / plane), per = std::max(1, std::min(target / (int)plane, planes));
   d.rows = per * (int)plane;
   d.threads = (d.rows + 31) / 32 * 32;

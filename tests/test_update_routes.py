@@ -98,12 +98,13 @@ DUO = [(4, (8, 4, 6, 6)), (4, (4, 8, 2, 2)), (4, (16, 16, 16, 16)), (4, (6, 10, 
 
 
 # four sites per thread: rows of one to sixteen quads, rows that cross warps (24, 40),
-# extents of 2, partly filled blocks, planes of up to 1024 threads; register bounds 96
+# extents of 2, partly filled blocks, blocks of 288 (the last), planes of up to 1024 threads; register bounds 96
 # (few blocks), 72 (64 x 64 x 4 x 2; several waves of 288 threads) and 64 (planes above
 # 896 threads; several waves of 512, links above half the L2)
 QUAD_DUO = [(4, (8, 2, 2, 2)), (4, (8, 4, 4, 6)), (4, (16, 16, 16, 16)), (4, (24, 24, 4, 6)), (4, (40, 40, 4, 4)),
             (4, (64, 64, 4, 2)), (4, (128, 64, 4, 4)), (4, (8, 4, 34, 34)), (4, (48, 48, 24, 20)),
-            (4, (64, 64, 24, 24)), (3, (16, 10, 0, 6)), (3, (32, 34, 0, 38))]
+            (4, (64, 64, 24, 24)), (3, (16, 10, 0, 6)), (3, (32, 34, 0, 38)), (4, (16, 24, 6, 4)), (4, (24, 16, 6, 4)),
+            (4, (24, 24, 6, 10))]
 
 
 def _duo_child(out, geometries=None):

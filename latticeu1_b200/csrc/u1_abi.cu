@@ -480,7 +480,7 @@ static int export_angles(u1_lattice *lat, double *angles, int on_device, bool wa
     if (rc) return rc;
     dst = lat->stage;
   }
-  k_export_angles<<<export_blocks(n), 256, 0, lat->stream>>>(lat->links, dst, n);
+  k_export_angles<<<u1i::blocks_for((long long)n, 256), 256, 0, lat->stream>>>(lat->links, dst, n);
   U1_LAUNCH_CHECK("k_export_angles");
   if (!on_device)
     U1_CUDA_TRY(cudaMemcpyAsync(angles, lat->stage, n * sizeof(double), cudaMemcpyDeviceToHost, lat->stream));

@@ -729,7 +729,7 @@ static int chain_io(u1_batch *b, int chain, double *host, bool import) {
       e = cudaGetLastError();
     }
   } else {
-    k_export_angles<<<export_blocks(n), 256, 0, b->stream>>>(ch.links, tmp, n);
+    k_export_angles<<<nblocks((long long)n, 256), 256, 0, b->stream>>>(ch.links, tmp, n);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(host, tmp, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
   }
@@ -744,7 +744,7 @@ extern "C" int u1_batch_export_all(u1_batch *b, double *angles_dev) {
   if (!b || !angles_dev) return bfail(U1_ERR_INVALID, "u1_batch_export_all: null argument");
   U1_CUDA_TRY(cudaSetDevice(b->ctx->device));
   // chains are stored back to back, so one elementwise pass converts them all
-  k_export_angles<<<export_blocks(b->total_links), 256, 0, b->stream>>>(b->links, angles_dev,
+  k_export_angles<<<nblocks((long long)b->total_links, 256), 256, 0, b->stream>>>(b->links, angles_dev,
                                                                                   b->total_links);
   U1_LAUNCH_CHECK("k_export_angles (batch)");
   return U1_OK;

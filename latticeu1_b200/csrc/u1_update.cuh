@@ -11,8 +11,6 @@
 // overrelaxation reflection theta' = -theta - 2 arg S becomes
 // U' = (conj S / |S|)^2 * conj U, with no transcendental call.
 #pragma once
-#include <algorithm>
-
 #include "u1_cplx.cuh"
 #include "u1_geom.cuh"
 #include "u1_philox.h"
@@ -830,71 +828,14 @@ static __global__ void k_import_angles(float2 *lat, const double *ang, size_t n)
   lat[i] = make_float2((float)c, (float)s);
 }
 
-// Angle in [0, 2 pi) of a link (x, y) on the unit circle (FP32 rounding), to FP64
-// rounding.  The octant's angle phi = atan(v / u), u >= v >= 0, is taken from the
-// nearest of nine directions phi_k = k pi / 32 (tab: cos, sin; phi):
-// t = tan(phi - phi_k) = (v c - u s) / (u c + v s) is at most 0.053, so six terms
-// of the arctangent's series reach 1e-17, and the denominator is within 0.01 of 1, so
-// its reciprocal is 2 - den after one Newton step and a correction of the
-// quotient.  About 20 FP64 operations and two conversions; the general atan2 made
-// the 512-chain export FP64-bound (783 us for 2.3 GB).
-struct AngleTable {
-  double2 cs[9];
-  double phi[9];
-};
-__device__ __forceinline__ double link_angle(float2 l, const AngleTable &tab) {
-  const float n2 = fmaf(l.x, l.x, l.y * l.y);
-  if (!(n2 > 0.99f && n2 < 1.01f)) {  // not a normalised link: the general function
-    double t = atan2((double)l.y, (double)l.x);
-    return t < 0.0 ? t + 6.283185307179586476925 : t;
-  }
-  const float ax = fabsf(l.x), ay = fabsf(l.y);
-  const float u = fmaxf(ax, ay), v = fminf(ax, ay), q = __fdividef(v, u);
-  // 32 / pi of the octant's angle to 0.04, rounded by adding 1.5 * 2^23
-  const int k = __float_as_int(fmaf(q * 10.1859164f, fmaf(-0.273f, q, 1.0583982f), 12582912.f)) & 15;
-  const double2 cs = tab.cs[k];
-  const double U = (double)u, V = (double)v;
-  const double num = fma(V, cs.x, -(U * cs.y)), den = fma(U, cs.x, V * cs.y);
-  double r = 2.0 - den;
-  r = fma(r, fma(-den, r, 1.0), r);
-  double t = num * r;
-  t = fma(fma(-den, t, num), r, t);
-  const double z = t * t;
-  double s = fma(z, -1.0 / 11.0, 1.0 / 9.0);
-  s = fma(z, s, -1.0 / 7.0);
-  s = fma(z, s, 1.0 / 5.0);
-  s = fma(z, s, -1.0 / 3.0);
-  double phi = tab.phi[k] + fma(t * z, s, t);
-  if (ay > ax) phi = 1.570796326794896619231 - phi;
-  if (l.x < 0.f) phi = 3.141592653589793238463 - phi;
-  if (l.y < 0.f) phi = 6.283185307179586476925 - phi;
-  return phi;
-}
-
-static __global__ void __launch_bounds__(256) k_export_angles(const float2 *__restrict__ lat, double *__restrict__ ang,
-                                                              size_t n) {
-  __shared__ AngleTable tab;
-  if (threadIdx.x < 9) {
-    double s, c;
-    sincospi(threadIdx.x * (1.0 / 32.0), &s, &c);
-    tab.cs[threadIdx.x] = make_double2(c, s);
-    tab.phi[threadIdx.x] = threadIdx.x * 0.09817477042468103870;
-  }
-  __syncthreads();
-  const size_t step = (size_t)gridDim.x * blockDim.x;
+static __global__ void k_export_angles(const float2 *lat, double *ang, size_t n) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + 3 * step < n; i += 4 * step) {  // four loads in flight
-    float2 l[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) l[k] = lat[i + k * step];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) ang[i + k * step] = link_angle(l[k], tab);
-  }
-  for (; i < n; i += step) ang[i] = link_angle(lat[i], tab);
+  if (i >= n) return;
+  float2 u = lat[i];
+  double t = atan2((double)u.y, (double)u.x);
+  if (t < 0.0) t += 2.0 * 3.14159265358979323846;
+  ang[i] = t;
 }
-
-// Blocks of k_export_angles: at most eight per SM, each building its table once.
-__host__ inline int export_blocks(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 8 * 148); }
 
 static __global__ void k_fill_links(float2 *lat, size_t n, float2 v) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;

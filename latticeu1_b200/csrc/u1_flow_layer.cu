@@ -181,7 +181,7 @@ __device__ __forceinline__ void stage_weights(const FlowK &f, float *w1, float *
     const int r = t / PADS, e = t - r * PADS;
     w2[r * WS + (e < 3 ? e * 2 * NP + C2 : 6 * NP + e - 3)] = 0.f;
   }
-#pragma unroll 4
+#pragma unroll 8
   for (int t = (int)threadIdx.x; t < C2 * H * 9; t += nt) {  // in memory order: o, channel, ky, kx
     const int oc = t / 9, k = t - 9 * oc, ky = k / 3, kx = k - 3 * ky;
     const int o = oc / H, c = oc - o * H;
@@ -707,12 +707,13 @@ __global__ void __launch_bounds__(1024) k_flow_wgrad_reduce(const float *__restr
   out[to] = v;
 }
 
+constexpr int kSms = 148;
+
 // Configurations per block, at most `pairs` plaquette pairs: the fewest pairs
 // on the busiest SM, a block's weight staging counted as 12 (batch 1024: one
 // configuration per block at L = 32, 7 blocks on the busiest SM; seven at L = 16,
 // one block per SM).
 int flow_nc(int L, int batch, int pairs) {
-  constexpr int kSms = 148;
   const int tp = L * L / 8;
   int best = 1;
   long long cost = -1;
@@ -740,7 +741,12 @@ void flow_pitches(FlowK &f) {
   f.dhp = u1b::make_fastdiv((uint32_t)(L / 2));
 }
 
-int flow_threads(const FlowK &f) { return (2 * f.nc * (f.L * f.L / 8) + 31) / 32 * 32; }
+// Two threads per pair, and at least `least`: the others help to stage the weights
+// and the context, which one warp alone takes longer over than over the sums (four
+// layers of 8^2, batch 126, a block of 16 threads' sums: 145 us with 32 threads).
+int flow_threads(const FlowK &f, int least) {
+  return std::max(least, (2 * f.nc * (f.L * f.L / 8) + 31) / 32 * 32);
+}
 
 template <int NP>
 size_t flow_weights_floats(int H) {
@@ -751,13 +757,14 @@ template <int NP, bool INV>
 int launch_forward(FlowK f, const char *name, cudaStream_t st) {
   f.nc = flow_nc(f.L, f.batch, kFwdThreads / 2);
   flow_pitches(f);
-  const int threads = flow_threads(f);
+  const int nb = (f.batch + f.nc - 1) / f.nc;
+  const int threads = flow_threads(f, nb <= kSms ? kFwdThreads : kFwdThreads / 2);
   const size_t work = std::max((size_t)3 * kChunk * f.rp, (size_t)2 * NP * threads);
   const size_t smem = sizeof(float) * (flow_weights_floats<NP>(f.H) + 4 * (size_t)f.cp + work);
   const cudaError_t e =
       cudaFuncSetAttribute(k_flow_forward<NP, INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return u1i::cuda_fail(e, name);
-  k_flow_forward<NP, INV><<<(f.batch + f.nc - 1) / f.nc, threads, smem, st>>>(f);
+  k_flow_forward<NP, INV><<<nb, threads, smem, st>>>(f);
   U1_LAUNCH_CHECK(name);
   return U1_OK;
 }
@@ -767,7 +774,7 @@ int launch_backward(FlowK f, const char *name, float *wgrad, cudaStream_t st) {
   using Dm = FlowDims<NP>;
   f.nc = flow_nc(f.L, f.batch, kBwdThreads / 2);
   flow_pitches(f);
-  const int LL = f.L * f.L, threads = flow_threads(f), nwarps = threads / 32;
+  const int LL = f.L * f.L, threads = flow_threads(f, kBwdThreads), nwarps = threads / 32;
   const size_t work = std::max({6 * (size_t)kChunk * f.rp, (size_t)nwarps * kChunk * (9 * Dm::GP + 20),
                                 (size_t)2 * NP * threads, (size_t)f.nc * LL});
   const size_t smem = sizeof(float) * (flow_weights_floats<NP>(f.H) + 4 * (size_t)f.cp +

@@ -442,8 +442,8 @@ int u1_flow_layer_backward(const float *theta_in, const float *grad_theta_out, c
  * u1_flow_layer_forward: the same context net (the context plaquettes hold no
  * updated link, so the layer and its inverse see the same parameters), then
  * the inverse mixture transform of each active plaquette (bracketed Newton
- * steps to the float resolution), the
- * link change that undoes a forward step, and logdet[b] = sum of log H' at the
+ * steps; the residual of the solution is within the FP32 rounding of the
+ * transform), the link change that undoes a forward step, and logdet[b] = sum of log H' at the
  * solutions (the forward layer's log-det at the returned configuration). */
 int u1_flow_layer_inverse(const float *theta_in, float *theta_out, float *logdet, int batch, int L, int mu, int off,
                           int K, int hidden, const float *W1, const float *B1, const float *W2, const float *B2,

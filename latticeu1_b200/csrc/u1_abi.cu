@@ -1724,21 +1724,33 @@ extern "C" int u1_multilevel(u1_lattice *lat, u1_rng *rng, int n4, int k4, int n
   // sub-updates, T2, T4: about 260 MB at 24^3 x 32) are allocated by the first
   // call and kept with the lattice, so later calls neither allocate nor
   // synchronise the device.  A batch is up to 16 sub-updates or 256 MiB of slab
-  // products; one sub-update where the device has no memory for a large batch.
+  // products; where the device has no memory for that beside T2 and T4, one
+  // sub-update, which needs what the tensors alone need.  (A batch of up to
+  // 2 MiB, one granule of cudaMalloc, is not given up: it cannot be what is missing.)
   if (!lat->ml_work) {
     float2 *work = nullptr;
     double2 *P2 = nullptr, *T2 = nullptr, *T4 = nullptr;
-    cudaError_t e = u1i::dev_alloc(&work, (size_t)g.V * g.dims * sizeof(float2));
     const size_t slab_bytes = (size_t)g.Vs * nl2 * sizeof(double2);
     int batch = (int)std::max<size_t>(1, std::min<size_t>(16, (256ull << 20) / slab_bytes));
-    if (e == cudaSuccess) e = u1i::dev_alloc(&P2, slab_bytes * batch);
-    if (e == cudaErrorMemoryAllocation && work && slab_bytes * batch > (32ull << 20) && batch > 1) {
-      cudaGetLastError();
-      batch = 1;
-      e = u1i::dev_alloc(&P2, slab_bytes);
+    auto tensors = [&]() {
+      cudaError_t r = u1i::dev_alloc(&P2, slab_bytes * batch);
+      if (r == cudaSuccess) r = u1i::dev_alloc(&T2, size * nl2 * sizeof(double2));
+      if (r == cudaSuccess) r = u1i::dev_alloc(&T4, size * nl4 * sizeof(double2));
+      return r;
+    };
+    cudaError_t e = u1i::dev_alloc(&work, (size_t)g.V * g.dims * sizeof(float2));
+    if (e == cudaSuccess) {
+      e = tensors();
+      if (e == cudaErrorMemoryAllocation && batch > 1 && slab_bytes * batch > (2ull << 20)) {
+        cudaGetLastError();
+        for (double2 **p : {&P2, &T2, &T4}) {
+          u1i::dev_free(*p);
+          *p = nullptr;
+        }
+        batch = 1;
+        e = tensors();
+      }
     }
-    if (e == cudaSuccess) e = u1i::dev_alloc(&T2, size * nl2 * sizeof(double2));
-    if (e == cudaSuccess) e = u1i::dev_alloc(&T4, size * nl4 * sizeof(double2));
     if (e != cudaSuccess) {
       u1i::dev_free(work);
       u1i::dev_free(P2);

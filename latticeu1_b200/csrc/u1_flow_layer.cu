@@ -753,6 +753,26 @@ size_t flow_weights_floats(int H) {
   return (size_t)20 * H + (size_t)3 * H * FlowDims<NP>::WS + 20;
 }
 
+// The largest shared memory of any legal shape, for a block of `pairs` plaquette
+// pairs, two threads each (kernels' comments: the parts): (L / 4)(L + 4) floats of
+// a plane hold L^2 / 8 pairs, so a plane is at most 4 pairs (L = 4).  Each launch
+// sets its kernel's limit to this, the same value whatever its own shape, so
+// that threads with other shapes cannot lower it between the setting and the launch.
+template <int NP>
+size_t flow_forward_smem_most() {
+  const size_t pairs = kFwdThreads / 2, plane = 4 * pairs;
+  return sizeof(float) * (flow_weights_floats<NP>(32) + 4 * (plane + 1) +
+                          std::max(3 * kChunk * (plane + 32), (size_t)2 * NP * kFwdThreads));
+}
+template <int NP>
+size_t flow_backward_smem_most() {
+  using Dm = FlowDims<NP>;
+  const size_t pairs = kBwdThreads / 2, plane = 4 * pairs;
+  return sizeof(float) * (flow_weights_floats<NP>(32) + 4 * (plane + 1) + 2 * pairs * Dm::GP +
+                          std::max({6 * kChunk * (plane + 32), (size_t)(kBwdThreads / 32) * kChunk * (9 * Dm::GP + 20),
+                                    (size_t)2 * NP * kBwdThreads, 8 * pairs}));
+}
+
 template <int NP, bool INV>
 int launch_forward(FlowK f, const char *name, cudaStream_t st) {
   f.nc = flow_nc(f.L, f.batch, kFwdThreads / 2);
@@ -762,7 +782,8 @@ int launch_forward(FlowK f, const char *name, cudaStream_t st) {
   const size_t work = std::max((size_t)3 * kChunk * f.rp, (size_t)2 * NP * threads);
   const size_t smem = sizeof(float) * (flow_weights_floats<NP>(f.H) + 4 * (size_t)f.cp + work);
   const cudaError_t e =
-      cudaFuncSetAttribute(k_flow_forward<NP, INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_flow_forward<NP, INV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)flow_forward_smem_most<NP>());
   if (e != cudaSuccess) return u1i::cuda_fail(e, name);
   k_flow_forward<NP, INV><<<nb, threads, smem, st>>>(f);
   U1_LAUNCH_CHECK(name);
@@ -780,7 +801,8 @@ int launch_backward(FlowK f, const char *name, float *wgrad, cudaStream_t st) {
   const size_t smem = sizeof(float) * (flow_weights_floats<NP>(f.H) + 4 * (size_t)f.cp +
                                        (size_t)f.nc * (LL / 4) * Dm::GP + work);
   const cudaError_t e =
-      cudaFuncSetAttribute(k_flow_backward<NP, INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_flow_backward<NP, INV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)flow_backward_smem_most<NP>());
   if (e != cudaSuccess) return u1i::cuda_fail(e, name);
   const int nb = (f.batch + f.nc - 1) / f.nc;
   k_flow_backward<NP, INV><<<nb, threads, smem, st>>>(f);

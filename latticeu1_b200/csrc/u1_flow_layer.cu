@@ -707,19 +707,25 @@ __global__ void __launch_bounds__(1024) k_flow_wgrad_reduce(const float *__restr
   out[to] = v;
 }
 
-constexpr int kSms = 148;
+int device_sms() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
+    return 148;
+  return n;
+}
 
 // Configurations per block, at most `pairs` plaquette pairs: the fewest pairs
 // on the busiest SM, a block's weight staging counted as 12 (batch 1024: one
 // configuration per block at L = 32, 7 blocks on the busiest SM; seven at L = 16,
 // one block per SM).
-int flow_nc(int L, int batch, int pairs) {
+int flow_nc(int L, int batch, int pairs, int sms) {
   const int tp = L * L / 8;
   int best = 1;
   long long cost = -1;
   for (int nc = 1; nc <= std::max(1, pairs / tp) && nc <= batch; ++nc) {
     const int blocks = (batch + nc - 1) / nc;
-    const long long c = (long long)((blocks + kSms - 1) / kSms) * (nc * tp + 12);
+    const long long c = (long long)((blocks + sms - 1) / sms) * (nc * tp + 12);
     if (cost < 0 || c < cost) {
       cost = c;
       best = nc;
@@ -775,10 +781,11 @@ size_t flow_backward_smem_most() {
 
 template <int NP, bool INV>
 int launch_forward(FlowK f, const char *name, cudaStream_t st) {
-  f.nc = flow_nc(f.L, f.batch, kFwdThreads / 2);
+  const int sms = device_sms();
+  f.nc = flow_nc(f.L, f.batch, kFwdThreads / 2, sms);
   flow_pitches(f);
   const int nb = (f.batch + f.nc - 1) / f.nc;
-  const int threads = flow_threads(f, nb <= kSms ? kFwdThreads : kFwdThreads / 2);
+  const int threads = flow_threads(f, nb <= sms ? kFwdThreads : kFwdThreads / 2);
   const size_t work = std::max((size_t)3 * kChunk * f.rp, (size_t)2 * NP * threads);
   const size_t smem = sizeof(float) * (flow_weights_floats<NP>(f.H) + 4 * (size_t)f.cp + work);
   const cudaError_t e =
@@ -793,7 +800,7 @@ int launch_forward(FlowK f, const char *name, cudaStream_t st) {
 template <int NP, bool INV>
 int launch_backward(FlowK f, const char *name, float *wgrad, cudaStream_t st) {
   using Dm = FlowDims<NP>;
-  f.nc = flow_nc(f.L, f.batch, kBwdThreads / 2);
+  f.nc = flow_nc(f.L, f.batch, kBwdThreads / 2, device_sms());
   flow_pitches(f);
   const int LL = f.L * f.L, threads = flow_threads(f, kBwdThreads), nwarps = threads / 32;
   const size_t work = std::max({6 * (size_t)kChunk * f.rp, (size_t)nwarps * kChunk * (9 * Dm::GP + 20),

@@ -149,7 +149,9 @@ int u1_tune(u1_lattice *lat, u1_rng *rng, int *variant);
 /* Threads per block of the phase kernels of variants 1, 2, 3, 5 (32, ..., 256;
  * default 256; the reference's block.x, include/tune.h:143-260).  Every block
  * size gives bit-identical links.  The measuring phases of a measured sweep
- * and the persistent variant keep their own block sizes. */
+ * and the persistent variant keep their own block sizes.  A lattice whose
+ * block size is set runs the phase kernels, one phase per launch, until
+ * u1_tune or u1_lattice_set_variant(lat, 0). */
 int u1_lattice_set_block(u1_lattice *lat, int threads);
 int u1_lattice_get_block(const u1_lattice *lat, int *threads);
 /* Device pointer of the float2 link array (V*dims float2). */

@@ -1453,6 +1453,7 @@ extern "C" int u1_lattice_set_block(u1_lattice *lat, int threads) {
     return fail(U1_ERR_INVALID, "u1_lattice_set_block: threads per block must be 32, 64, ..., 256");
   lat->block = threads;
   lat->duo = false;  // an explicit block size is for one phase per launch
+  lat->explicit_variant = true;
   drop_graphs(lat);
   return U1_OK;
 }

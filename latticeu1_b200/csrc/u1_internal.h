@@ -99,7 +99,7 @@ struct u1_lattice {
   bool use_graphs = true;
   int variant = U1V_AUTO;          // update kernel variant (U1V_AUTO: tune on first update)
   int block = 256;                 // threads per block of the phase kernels (tuned with the variant)
-  bool explicit_variant = false;   // set by u1_lattice_set_variant (else chosen automatically)
+  bool explicit_variant = false;   // a variant or block size was set (else chosen automatically)
   bool duo = false;                // two phases per launch, chosen by the tuner with U1V_SINGLE (u1_duo.cuh) or U1V_QUAD (u1_quad_duo.cu)
   int cluster_ok = -1;             // sweeps as one cluster launch: -1 unknown, 0 no, 1 yes (layout: cluster)
   u1b::ClusterK cluster{};

@@ -114,7 +114,12 @@ int u1_lattice_set_graphs(u1_lattice *lat, int enable);
  * (4D, (Nx/2)*Ny/2 a multiple of 32 in [64, 256], every (z, t) tile resident
  * at once; opt-in, slower than 1 on B200 at 32^4). */
 int u1_lattice_set_variant(u1_lattice *lat, int variant);
-/* The variant in use: 0 while automatic and not yet tuned. */
+/* The variant in use: 0 while automatic and before the first update.  Of a
+ * lattice whose sweeps are one cluster launch: the default variant, for what
+ * still runs phase by phase (u1_update_phase, replayed proposals).  Setting it
+ * on another lattice does not copy what the automatic choice holds beside it
+ * (the cluster launch, two phases per launch): leave that lattice automatic,
+ * tuned choices are cached per geometry. */
 int u1_lattice_get_variant(const u1_lattice *lat, int *variant);
 /* Waits of the persistent sweep (variant 4; no counterpart in the reference):
  * each neighbour wait polls at most spin_limit times (0: the default, about a
@@ -151,7 +156,8 @@ int u1_tune(u1_lattice *lat, u1_rng *rng, int *variant);
  * size gives bit-identical links.  The measuring phases of a measured sweep
  * and the persistent variant keep their own block sizes.  A lattice whose
  * block size is set runs the phase kernels, one phase per launch, until
- * u1_tune or u1_lattice_set_variant(lat, 0). */
+ * u1_tune or u1_lattice_set_variant(lat, 0); before the first update of an
+ * automatic lattice it is replaced by that update's tuning. */
 int u1_lattice_set_block(u1_lattice *lat, int threads);
 int u1_lattice_get_block(const u1_lattice *lat, int *threads);
 /* Device pointer of the float2 link array (V*dims float2). */

@@ -1489,11 +1489,15 @@ static int update_impl(u1_lattice *lat, u1_rng *rng, int metrop, int ovrn, doubl
   int rc = check_replay(lat, rng, metrop);
   if (rc) return rc;
   const bool replay = rng->replay_dev != nullptr;
+  const bool cluster = cluster_usable(lat, metropolis_src(lat, rng));  // worked out before a capture
   if (lat->variant == U1V_AUTO && !replay && tuning_enabled()) {
-    rc = tune_update(lat, rng, true);
-    if (rc) return rc;
+    if (cluster) {  // nothing to tune; the default kernel takes what stays phase by phase
+      lat->variant = default_variant(lat->g);
+    } else {
+      rc = tune_update(lat, rng, true);
+      if (rc) return rc;
+    }
   }
-  cluster_usable(lat, metropolis_src(lat, rng));  // worked out before a capture
   if (lat->use_graphs && !replay && sweep_variant(lat, metropolis_src(lat, rng), 0) != U1V_WAVE) {
     // graph key: passes, rng object, seed/chain and whether the last pass measures
     auto key = std::make_tuple(metrop * 2 + (meas_partials ? 1 : 0), ovrn, rng->id,

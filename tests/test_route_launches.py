@@ -57,3 +57,24 @@ def test_block_size_selects_the_phase_kernels(ctx, monkeypatch):
     lat.tune(rng)  # gives the choice back
     assert _launches(lat, rng) == 1
     lat.close()
+
+
+@pytest.mark.parametrize("dims,N,tuned", [(4, (8, 8, 8, 8), False), (2, (32, 0, 0, 32), False),
+                                          (4, (16, 16, 16, 16), True)])
+def test_only_phase_kernels_are_tuned(ctx, dims, N, tuned, monkeypatch, tmp_path):
+    """The first update of a lattice on the cluster route times nothing: no trial, no line in the cache."""
+    from latticeu1_b200 import Lattice, Rng
+    monkeypatch.setenv("U1_RESOURCE_PATH", str(tmp_path))
+    monkeypatch.delenv("U1_TUNE", raising=False)
+    monkeypatch.delenv("U1_CLUSTER", raising=False)
+    lat, rng = Lattice(ctx, dims, N, 1.1), Rng(ctx, 5)
+    lat.hot_start(rng)
+    n = _launches(lat, rng)
+    lines = [p.read_text() for p in tmp_path.glob("u1b200_tunecache.tsv")]
+    if tuned:
+        # another test of this process may have tuned the geometry already: then it is taken from memory
+        assert n > 1 and len(lines) <= 1
+    else:
+        assert n == 1 and not lines
+    assert lat.variant in (1, 2, 3, 5)
+    lat.close()

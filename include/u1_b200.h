@@ -474,14 +474,20 @@ int u1_kernel_launch_count(uint64_t *out);
  * never performed.  After every phase a kernel counts the links that were
  * written and also read by another thread, or written twice, in that phase
  * (checkerboard races; not for the persistent variant 4, whose phases
- * overlap within one launch).
+ * overlap within one launch).  Of a launch of two phases the link's block
+ * is recorded too: a link that two blocks read or write and one of them
+ * writes is a race.  The one-launch cluster sweep runs in the checked build
+ * only with U1_CLUSTER=1; its shared-memory addresses are checked, and no
+ * phases are counted.
  * u1_check_report: out[0] violations, out[1] races, out[2] phases checked,
  * out[3] links accessed (summed over the phases), out[4..6] index, half size
- * and kind (0 read, 1 own read, 2 write) of the first violation (-1: none),
+ * and kind (0 read, 1 own read, 2 write, 3 read of a link that the same
+ * launch stores later) of the first violation (-1: none),
  * out[7] a raced link's buffer offset (-1: none); synchronises the device;
  * reset != 0 clears the counters.  u1_check_selftest runs the checks on a
  * 16-link slab with two refused accesses and two races planted in the marks
- * (never dereferenced) and reports as u1_check_report.  In the normal build
+ * (never dereferenced) and reports as u1_check_report; it fails where links
+ * claimed by two blocks, planted in a second run, are not found.  In the normal build
  * both return U1_ERR_UNSUPPORTED. */
 int u1_check_report(u1_ctx *ctx, int64_t out[8], int reset);
 int u1_check_selftest(u1_ctx *ctx, int64_t out[8]);

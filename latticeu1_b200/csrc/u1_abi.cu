@@ -333,7 +333,7 @@ extern "C" int u1_lattice_create(u1_ctx *ctx, const u1_geom *geom, u1_lattice **
     return U1_ERR_NOMEM;
   }
 #ifdef U1_BOUNDS_CHECK
-  lat->shadow = u1i::chk_shadow(nl);
+  lat->shadow = u1i::chk_shadow(2 * nl);
   if (!lat->shadow || !u1i::chk_state(ctx)) {
     u1_lattice_destroy(lat);
     return fail(U1_ERR_NOMEM, "u1_lattice_create: no device memory for the access checks");
@@ -935,17 +935,17 @@ static cudaLaunchConfig_t cluster_config(const u1_lattice *lat, cudaLaunchAttrib
 // and the gain is gone at about 700 sites per block (12^4, 648: 73.9 us
 // against 86.2), so larger 4D lattices keep the phase kernels; 2D and 3D
 // lattices use all 1024 threads (3D 32^3: 45.0 against 51.3).
-// U1_CLUSTER=0 in the environment turns it off; the checked build checks the
-// phase kernels.
+// U1_CLUSTER=0 in the environment turns it off; the checked build takes it only
+// with U1_CLUSTER=1 (shared-memory addresses are checked, phases are not counted).
 static bool cluster_usable(u1_lattice *lat, int src) {
-#ifdef U1_BOUNDS_CHECK
-  return false;
-#endif
   if (lat->explicit_variant || src == SRC_REPLAY) return false;
   if (lat->cluster_ok < 0) {
     lat->cluster_ok = 0;
     const char *env = std::getenv("U1_CLUSTER");
     const GeomK &g = lat->g;
+#ifdef U1_BOUNDS_CHECK
+    if (!env || env[0] != '1') return false;
+#endif
     if (env && env[0] == '0') return false;
     if (!cluster_layout(g, g.Vh <= 512 ? 1 : kClusterBlocks, lat->cluster)) return false;
     if (g.dims == 4 && lat->cluster.threads > 704) return false;
@@ -1090,6 +1090,7 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
 #ifdef U1_BOUNDS_CHECK
   a.chk = lat->ctx->chk;
   a.shadow = lat->shadow;
+  a.owner = lat->shadow + (size_t)lat->g.dims * lat->g.V;
   a.chk_base = links;
 #endif
   const int src = metropolis_src(lat, rng);
@@ -1144,7 +1145,7 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
       }
       ++a.mu;
 #ifdef U1_BOUNDS_CHECK
-      if (rc == U1_OK) rc = u1i::chk_phase_end(lat->stream, a.shadow, (size_t)D * lat->g.V, a.chk);
+      if (rc == U1_OK) rc = u1i::chk_phase_end(lat->stream, a.shadow, a.owner, (size_t)D * lat->g.V, a.chk);
 #endif
       return rc;
     }
@@ -1162,7 +1163,7 @@ static int issue_sweep(u1_lattice *lat, float2 *links, u1_rng *rng, int metrop, 
          : D == 3 ? launch_phase<3>(a, lat->stream, met, src, var, lat->block)
                   : launch_phase<4>(a, lat->stream, met, src, var, lat->block);
 #ifdef U1_BOUNDS_CHECK
-    if (rc == U1_OK) rc = u1i::chk_phase_end(lat->stream, a.shadow, (size_t)D * lat->g.V, a.chk);
+    if (rc == U1_OK) rc = u1i::chk_phase_end(lat->stream, a.shadow, a.owner, (size_t)D * lat->g.V, a.chk);
 #endif
     return rc;
   };
@@ -1597,7 +1598,7 @@ extern "C" int u1_update_phase(u1_lattice *lat, u1_rng *rng, int metropolis, int
     default: rc = launch_phase<4>(a, lat->stream, met, src, var, lat->block); break;
   }
 #ifdef U1_BOUNDS_CHECK
-  if (rc == U1_OK) rc = u1i::chk_phase_end(lat->stream, a.shadow, (size_t)lat->g.dims * lat->g.V, a.chk);
+  if (rc == U1_OK) rc = u1i::chk_phase_end(lat->stream, a.shadow, nullptr, (size_t)lat->g.dims * lat->g.V, a.chk);
 #endif
   return rc;
 }

@@ -619,7 +619,7 @@ static int batch_issue_sweep(u1_batch *b, int metrop, int ovrn, bool measure, in
              : D == 3 ? batch_phase<3>(b, ph, mu, met, grp, s)
                       : batch_phase<4>(b, ph, mu, met, grp, s);
 #ifdef U1_BOUNDS_CHECK
-      if (rc == U1_OK) rc = u1i::chk_phase_end(s, ph.shadow + g_off, g_len, ph.chk);
+      if (rc == U1_OK) rc = u1i::chk_phase_end(s, ph.shadow + g_off, nullptr, g_len, ph.chk);
 #endif
       return rc;
     };

@@ -23,16 +23,18 @@ int fail(int code, const std::string &msg) {
 
 #ifdef U1_BOUNDS_CHECK
 // After one phase: a link with a write mark (>= 2) that another thread also
-// read (bit 0), or with two writes (>= 4), is a race.  Counts the races and
-// the marked links, clears the marks and counts the phase.
-__global__ void __launch_bounds__(256) k_chk_phase_end(unsigned *shadow, size_t n, ChkState *st) {
+// read (bit 0), with two writes (>= 4), or that two blocks claim, is a race.
+// Counts the races and the marked links, clears the marks and owners and counts
+// the phase.
+__global__ void __launch_bounds__(256) k_chk_phase_end(unsigned *shadow, unsigned *owner, size_t n, ChkState *st) {
   unsigned long long races = 0, marked = 0;
   long long first = -1;
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
-    const unsigned w = shadow[k];
+    const unsigned w = shadow[k], n_w = w & ~u1b::kChkTwoBlocks;
+    if (owner != nullptr && owner[k] != 0u) owner[k] = 0u;
     if (w == 0u) continue;
     ++marked;
-    if (w >= 4u || (w >= 2u && (w & 1u))) {
+    if (n_w >= 4u || (n_w >= 2u && (w != n_w || (w & 1u)))) {
       ++races;
       if (first < 0) first = (long long)k;
     }
@@ -50,7 +52,7 @@ __global__ void __launch_bounds__(256) k_chk_phase_end(unsigned *shadow, size_t 
 // and two clean links (7 read by two threads, 9 read and written by its
 // owner).  One warp, one lane per access.
 __global__ void k_chk_selftest(const float2 *slab, unsigned *shadow, ChkState *st) {
-  const u1b::Chk c{st, shadow, slab, 16};
+  const u1b::Chk c{st, shadow, slab, 16, nullptr};
   switch (threadIdx.x) {
     case 0: u1b::chk<4, u1b::CHK_READ>(c, slab, 14); break;  // 14 + 4 > 16
     case 1: u1b::chk<2, u1b::CHK_READ>(c, slab, 1); break;   // 8-byte offset, 16-byte access
@@ -62,6 +64,23 @@ __global__ void k_chk_selftest(const float2 *slab, unsigned *shadow, ChkState *s
     case 7: u1b::chk<1, u1b::CHK_READ>(c, slab, 7); break;
     case 8: u1b::chk<1, u1b::CHK_OWN>(c, slab, 9); break;
     case 9: u1b::chk<1, u1b::CHK_WRITE>(c, slab, 9); break;
+    default: break;
+  }
+}
+
+// The same for the owners: link 3 read by block 0 and written by block 1, link 9
+// read by both and written by block 0 (two races); link 5 read and written by
+// block 0, link 7 read by both and not written (clean).
+__global__ void k_chk_selftest_blocks(const float2 *slab, unsigned *shadow, unsigned *owner, ChkState *st) {
+  const u1b::Chk c{st, shadow, slab, 16, owner};
+  const bool first = blockIdx.x == 0;
+  switch (threadIdx.x) {
+    case 0: first ? u1b::chk<1, u1b::CHK_LIVE>(c, slab, 3) : u1b::chk<1, u1b::CHK_WRITE>(c, slab, 3); break;
+    case 1: if (first) u1b::chk<1, u1b::CHK_LIVE>(c, slab, 5); break;
+    case 2: if (first) u1b::chk<1, u1b::CHK_WRITE>(c, slab, 5); break;
+    case 3: u1b::chk<1, u1b::CHK_LIVE>(c, slab, 7); break;
+    case 4: u1b::chk<1, u1b::CHK_LIVE>(c, slab, 9); break;
+    case 5: if (first) u1b::chk<1, u1b::CHK_WRITE>(c, slab, 9); break;
     default: break;
   }
 }
@@ -117,16 +136,17 @@ unsigned *chk_shadow(size_t n) {
 #endif
 }
 
-int chk_phase_end(cudaStream_t s, unsigned *shadow, size_t n, ChkState *st) {
+int chk_phase_end(cudaStream_t s, unsigned *shadow, unsigned *owner, size_t n, ChkState *st) {
 #ifdef U1_BOUNDS_CHECK
   if (!shadow || !st) return U1_OK;
   const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 8);
-  k_chk_phase_end<<<blocks, 256, 0, s>>>(shadow, n, st);
+  k_chk_phase_end<<<blocks, 256, 0, s>>>(shadow, owner, n, st);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_chk_phase_end");
 #else
   (void)s;
   (void)shadow;
+  (void)owner;
   (void)n;
   (void)st;
 #endif
@@ -162,8 +182,8 @@ extern "C" int u1_check_selftest(u1_ctx *ctx, int64_t out[8]) {
   if (!ctx || !out) return fail(U1_ERR_INVALID, "u1_check_selftest: null argument");
 #ifdef U1_BOUNDS_CHECK
   U1_CUDA_TRY(cudaSetDevice(ctx->device));
-  // one allocation: the counters, 16 shadow words, then the 16-link slab
-  // (256-byte aligned from the allocator, so the slab is 16-byte aligned)
+  // one allocation: the counters, 16 shadow and 16 owner words, then the 16-link
+  // slab (256-byte aligned from the allocator, so the slab is 16-byte aligned)
   char *buf = nullptr;
   const size_t off_shadow = 256, off_slab = 512, bytes = 512 + 16 * sizeof(float2);
   U1_CUDA_TRY(u1i::dev_alloc(&buf, bytes));
@@ -179,14 +199,33 @@ extern "C" int u1_check_selftest(u1_ctx *ctx, int64_t out[8]) {
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
-    k_chk_phase_end<<<1, 256>>>(shadow, 16, st);
+    k_chk_phase_end<<<1, 256>>>(shadow, nullptr, 16, st);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
-  ChkState h{};
+  ChkState h{}, hb{};
   if (e == cudaSuccess) e = cudaMemcpy(&h, st, sizeof(h), cudaMemcpyDeviceToHost);
+  // the owners, counted apart
+  unsigned *owner = shadow + 16;
+  unsigned left[32];
+  if (e == cudaSuccess) e = cudaMemcpy(buf, &z, sizeof(z), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    k_chk_selftest_blocks<<<2, 32>>>(slab, shadow, owner, st);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) {
+    k_chk_phase_end<<<1, 256>>>(shadow, owner, 16, st);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e == cudaSuccess) e = cudaMemcpy(&hb, st, sizeof(hb), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(left, shadow, sizeof(left), cudaMemcpyDeviceToHost);
   u1i::dev_free(buf);
   if (e != cudaSuccess) return u1i::cuda_fail(e, "u1_check_selftest");
+  if (hb.bad != 0 || hb.races != 2 || hb.marked != 4 || hb.phases != 1 ||
+      (hb.first_race_link != 3 && hb.first_race_link != 9) ||
+      std::any_of(left, left + 32, [](unsigned w) { return w != 0u; }))
+    return fail(U1_ERR_INVALID, "u1_check_selftest: a link claimed by two blocks is not reported");
   report(h, out);
   return U1_OK;
 #else

@@ -113,6 +113,29 @@ __device__ __forceinline__ void cluster_pass(const UpdArgs &a, const ClusterSite
   }
 }
 
+// Checked build: whether r0 + step is the first site of one of the lattice's rows
+// (which cluster_layout gives a block and a place in it), and whether the four
+// steps along x0 stay in the row.  A violation is counted and not followed; with
+// the thread's own link these are all the addresses of a sweep.
+__device__ __forceinline__ bool chk_row(const Chk &c, int r0, int step, int hN0) {
+#ifdef U1_BOUNDS_CHECK
+  const int r = r0 + step;
+  return chk_count(c, r >= 0 && r < c.Vh && r % hN0 == 0, r);
+#else
+  return true;
+#endif
+}
+__device__ __forceinline__ bool chk_in_row(const Chk &c, int ko, const int (&df)[2], const int (&db)[2], int bytes) {
+#ifdef U1_BOUNDS_CHECK
+  bool ok = true;
+  for (int p = 0; p < 2; ++p)
+    ok = ok && ko + df[p] >= 0 && ko + df[p] < bytes && ko + db[p] >= 0 && ko + db[p] < bytes;
+  return chk_count(c, ok, ko / 8);
+#else
+  return true;
+#endif
+}
+
 template <int D, int SRC, bool ONE>
 __global__ void __launch_bounds__(kClusterThreads, 1)
     k_sweep_cluster(const UpdArgs a, const ClusterK c, int metrop, int ovrn, unsigned long long *pass_rw) {
@@ -137,14 +160,16 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     s.db[0] = odd0 ? 0 : kb;
     s.db[1] = odd0 ? kb : 0;
     const int r0 = (s.live ? s.i : 0) - k;  // EO index of the row's first site
+    const Chk ck = make_chk(a);
     auto at = [&](int step) -> uint32_t {   // address of the row r0 + step
-      const uint32_t row = fast_div((uint32_t)(r0 + step), g.fd[0]);
+      const uint32_t row = chk_row(ck, r0, step, g.hN0) ? fast_div((uint32_t)(r0 + step), g.fd[0]) : 0u;
       const uint32_t owner = ONE ? 0u : fast_div(row, c.fr);
       const uint32_t off = (row - owner * (uint32_t)c.rows) * (uint32_t)(g.hN0 * 8);
       return ONE ? base + off : cluster_map(base + off, (int)owner);
     };
     s.row = at(0);
     s.own = base + (uint32_t)t * 8u;
+    if (!chk_in_row(ck, s.ko, s.df, s.db, g.hN0 * 8)) s.df[0] = s.df[1] = s.db[0] = s.db[1] = 0;
 #pragma unroll
     for (int mu = 1; mu < D; ++mu) {
       s.up[mu] = at(fwd[mu]) + (uint32_t)s.ko;

@@ -126,7 +126,7 @@ struct u1_lattice {
   unsigned long long ml_n4 = 0, ml_n2 = 0;  // kernels per replay
   unsigned wave_spin_limit = 0;    // polls per neighbour wait (0: the kernel's default)
   int wave_stall_tile = -1;        // test hook: this tile never publishes its phases (-1: none)
-  unsigned *shadow = nullptr;      // checked build: per-link access marks (V*dims words)
+  unsigned *shadow = nullptr;      // checked build: per-link access marks, then owners (2 V*dims words)
 };
 
 namespace u1i {
@@ -169,9 +169,9 @@ inline cudaError_t dev_alloc(T **p, size_t bytes) {
 // first use) and a zeroed shadow of n words; elsewhere both return null.
 u1b::ChkState *chk_state(u1_ctx *ctx);
 unsigned *chk_shadow(size_t n);
-// Checked build: the race check and reset of the shadow after one phase on
-// stream s (no-op when shadow is null or in the normal build).
-int chk_phase_end(cudaStream_t s, unsigned *shadow, size_t n, u1b::ChkState *st);
+// Checked build: the race check and reset of the shadow and owners (may be null)
+// after one phase on stream s (no-op when shadow is null or in the normal build).
+int chk_phase_end(cudaStream_t s, unsigned *shadow, unsigned *owner, size_t n, u1b::ChkState *st);
 // Geometry from the ABI struct (Grid mapping of the reference's
 // SetupLatticeParameters); U1_ERR_INVALID on odd extents.
 int make_geom(const u1_geom *geom, u1b::GeomK &g);

@@ -96,6 +96,7 @@ struct UpdArgs {
 #ifdef U1_BOUNDS_CHECK
   struct ChkState *chk;                // checked build: violation counters (see Chk below)
   unsigned *shadow;                    // checked build: per-link marks of this phase (nullptr: no race marks)
+  unsigned *owner;                     // checked build: per-link block of a launch of two phases (nullptr: not recorded)
   const float2 *chk_base;              // checked build: the link buffer the shadow mirrors
 #endif
 };
@@ -112,8 +113,13 @@ struct UpdArgs {
 // bit 0 for a read of a link the thread does not own, +2 for a write.
 // k_chk_phase_end runs after every launch: a link written and also read by
 // another thread, or written twice, within one phase is a checkerboard race;
-// it counts them and clears the marks.  In the normal build Chk is empty and
-// every check folds to `true`.
+// it counts them and clears the marks.  In a launch of two phases a thread also
+// reads, before a block barrier, links that another thread of its block stores
+// after it (CHK_LIVE).  That is sound only within a block, so the owner array
+// (one word per link) takes the block of every such read and of every store: a
+// link that two blocks claim and one of them stores is a race as well.  In the
+// normal build Chk is empty and every check folds to `true`.
+constexpr unsigned kChkTwoBlocks = 0x80000000u;  // in a link's mark: claimed by two blocks
 struct ChkState {
   unsigned long long bad;        // bounds or alignment violations
   unsigned long long races;      // links written and read (or written twice) within one phase
@@ -132,16 +138,17 @@ struct Chk {
   unsigned *shadow;
   const float2 *base;
   int Vh;
+  unsigned *owner;
 #endif
 };
 
 // another thread's link / the thread's own / a store / a link that a thread of
-// the same block stores later in the launch, after a barrier (no race mark)
+// the same block stores later in the launch, after a barrier
 enum : int { CHK_READ = 0, CHK_OWN = 1, CHK_WRITE = 2, CHK_LIVE = 3 };
 
 __device__ __forceinline__ Chk make_chk(const UpdArgs &a) {
 #ifdef U1_BOUNDS_CHECK
-  return Chk{a.chk, a.shadow, a.chk_base, a.g.Vh};
+  return Chk{a.chk, a.shadow, a.chk_base, a.g.Vh, a.owner};
 #else
   (void)a;
   return Chk{};
@@ -151,6 +158,22 @@ __device__ __forceinline__ Chk make_chk(const UpdArgs &a) {
 // Callers outside the update bodies (the standalone measurement) are not checked.
 __device__ __forceinline__ Chk no_chk() { return Chk{}; }
 
+// Counts a violation in the checked build; returns ok.
+__device__ __forceinline__ bool chk_count(const Chk &c, bool ok, int idx, int kind = CHK_READ) {
+#ifdef U1_BOUNDS_CHECK
+  if (!ok && c.st != nullptr && atomicAdd(&c.st->bad, 1ull) == 0ull) {
+    c.st->first_bad_idx = idx;
+    c.st->first_bad_half = c.Vh;
+    c.st->first_bad_kind = kind;
+  }
+#else
+  (void)c;
+  (void)idx;
+  (void)kind;
+#endif
+  return ok;
+}
+
 // Whether W consecutive links at slab[idx] may be accessed (always true in
 // the normal build); marks them in the checked build.
 template <int W, int KIND>
@@ -158,14 +181,7 @@ __device__ __forceinline__ bool chk(const Chk &c, const float2 *slab, int idx) {
 #ifdef U1_BOUNDS_CHECK
   if (c.st == nullptr) return true;  // an unchecked caller (no_chk)
   const bool ok = idx >= 0 && idx + W <= c.Vh && ((uintptr_t)(slab + idx) & (uintptr_t)(W * 8 - 1)) == 0;
-  if (!ok) {
-    if (atomicAdd(&c.st->bad, 1ull) == 0ull) {
-      c.st->first_bad_idx = idx;
-      c.st->first_bad_half = c.Vh;
-      c.st->first_bad_kind = KIND;
-    }
-    return false;
-  }
+  if (!chk_count(c, ok, idx, KIND)) return false;
   if (c.shadow != nullptr && KIND != CHK_OWN && KIND != CHK_LIVE) {
     unsigned *m = c.shadow + ((slab + idx) - c.base);
 #pragma unroll
@@ -174,6 +190,15 @@ __device__ __forceinline__ bool chk(const Chk &c, const float2 *slab, int idx) {
         atomicOr(m + k, 1u);
       else
         atomicAdd(m + k, 2u);
+    }
+  }
+  if (c.shadow != nullptr && c.owner != nullptr && (KIND == CHK_LIVE || KIND == CHK_WRITE)) {
+    const ptrdiff_t at = (slab + idx) - c.base;
+    const unsigned block = (unsigned)blockIdx.x + 1u;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const unsigned before = atomicCAS(c.owner + at + k, 0u, block);
+      if (before != 0u && before != block) atomicOr(c.shadow + at + k, kChkTwoBlocks);
     }
   }
   return true;

@@ -7,7 +7,17 @@ phases per launch: per half-pass 2 of 4 launches (4D) where both pairs of
 directions fit a block, 3 where one does, 2 of 3 in 3D."""
 from __future__ import annotations
 
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+for p in (ROOT, ROOT / "tests"):
+    if str(p) not in sys.path:
+        sys.path.insert(0, str(p))
 
 pytestmark = pytest.mark.gpu
 
@@ -19,15 +29,42 @@ def _launches(lat, rng, metrop=1, ovrn=2):
     return launch_count() - n
 
 
-# the smallest lattices, one block and sixteen, the largest of the route, and the
-# first ones beyond it (None): 1024 sites a block in 2D and 3D, 704 in 4D
-@pytest.mark.parametrize("dims,N,cluster", [
-    (2, (4, 0, 0, 4), True), (2, (32, 0, 0, 32), True), (2, (34, 0, 0, 32), True), (2, (128, 0, 0, 256), True),
-    (2, (130, 0, 0, 256), False), (3, (2, 2, 0, 2), True), (3, (32, 32, 0, 32), True), (3, (32, 34, 0, 32), False),
-    (4, (2, 2, 2, 2), True), (4, (8, 8, 8, 8), True), (4, (10, 12, 14, 12), True), (4, (22, 8, 8, 16), True),
-    (4, (12, 12, 12, 14), False)])
+# the smallest lattices, one block and sixteen, the largest of the route: 1024
+# sites a block in 2D and 3D, 704 in 4D
+CLUSTER = [(2, (4, 0, 0, 4), 1), (2, (32, 0, 0, 32), 1), (2, (34, 0, 0, 32), 1), (2, (62, 0, 0, 46), 1),
+           (2, (128, 0, 0, 256), 1), (3, (2, 2, 0, 2), 1), (3, (10, 6, 0, 14), 1), (3, (32, 32, 0, 32), 1),
+           (4, (2, 2, 2, 2), 1), (4, (8, 8, 8, 8), 1), (4, (6, 10, 8, 4), 1), (4, (10, 12, 14, 12), 1),
+           (4, (22, 8, 8, 16), 1)]
+# and the first ones beyond it
+BEYOND = [(2, (130, 0, 0, 256), 12), (3, (32, 34, 0, 32), 18), (4, (12, 12, 12, 14), 24)]
+
+# the geometries of test_update_routes with the launches of a half-pass, one and
+# four sites per thread: directions 2, 3 pair up in no four-site launch, and with
+# one site where diagonals of lcm(N2, N3) sites, eight or more side by side, fit 256 threads
+DUO_LAUNCHES = [2, 2, 2, 2, 3, 2, 2, 3, 2, 2, 2]
+QUAD_DUO_LAUNCHES = [3] * 10 + [2, 2] + [3] * 3
+
+
+def half_pass_launches(route):
+    import test_update_routes as t
+    geometries, counts = (t.DUO, DUO_LAUNCHES) if route == "duo" else (t.QUAD_DUO, QUAD_DUO_LAUNCHES)
+    assert len(geometries) == len(counts)
+    return [(dims, N, n) for (dims, N), n in zip(geometries, counts)]
+
+
+def cache_lines(route):
+    """A tune-cache file that names two phases per launch for every geometry of the route."""
+    import torch
+    name, variant, lines = torch.cuda.get_device_name(0), 3 if route == "duo" else 5, []
+    for k, (dims, N, _) in enumerate(half_pass_launches(route)):
+        g = {3: (N[0], N[1], N[3], 1), 4: N}[dims]
+        lines.append(f"{name}|update|{dims}|{'x'.join(map(str, g))}\t{variant}\t1.0\t{(128, 192, 256)[k % 3]}\t1\n")
+    return "".join(lines)
+
+
+@pytest.mark.parametrize("dims,N,launches", CLUSTER + BEYOND)
 @pytest.mark.parametrize("window", [None, (0.7, 3)])
-def test_cluster_route_is_taken(ctx, dims, N, cluster, window, monkeypatch):
+def test_cluster_route_is_taken(ctx, dims, N, launches, window, monkeypatch):
     from latticeu1_b200 import Lattice, Rng
     monkeypatch.setenv("U1_TUNE", "0")
     monkeypatch.delenv("U1_CLUSTER", raising=False)
@@ -36,7 +73,7 @@ def test_cluster_route_is_taken(ctx, dims, N, cluster, window, monkeypatch):
         lat.set_metropolis(*window)
     lat.hot_start(rng)
     for _ in range(2):
-        assert _launches(lat, rng) == (1 if cluster else 2 * dims * 3)
+        assert _launches(lat, rng) == launches
     lat.close()
 
 
@@ -78,3 +115,26 @@ def test_only_phase_kernels_are_tuned(ctx, dims, N, tuned, monkeypatch, tmp_path
         assert n == 1 and not lines
     assert lat.variant in (1, 2, 3, 5)
     lat.close()
+
+
+def _child(route):
+    from latticeu1_b200 import Context, Lattice, Rng
+    ctx = Context(0)
+    for dims, N, per in half_pass_launches(route):
+        lat, rng = Lattice(ctx, dims, N, 0.8), Rng(ctx, 3)
+        lat.hot_start(rng)
+        for _ in range(2):
+            n = _launches(lat, rng)
+            assert n == per * 2 * 3, (dims, N, n, per)
+        lat.close()
+    print("LAUNCHES_OK")
+
+
+@pytest.mark.parametrize("route", ["duo", "quad"])
+def test_two_phases_per_launch_are_launched(route, tmp_path):
+    (tmp_path / "u1b200_tunecache.tsv").write_text(cache_lines(route))
+    env = dict(os.environ, PYTHONPATH=f"{ROOT}:{ROOT / 'tests'}", U1_RESOURCE_PATH=str(tmp_path), U1_CLUSTER="0")
+    env.pop("U1_TUNE", None)
+    r = subprocess.run([sys.executable, "-c", f"import test_route_launches as t; t._child({route!r})"], env=env,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "LAUNCHES_OK" in r.stdout, (r.stdout[-3000:], r.stderr[-3000:])

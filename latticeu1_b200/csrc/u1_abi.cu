@@ -926,18 +926,39 @@ static cudaLaunchConfig_t cluster_config(const u1_lattice *lat, cudaLaunchAttrib
   return cfg;
 }
 
+// Sites of a block up to which the cluster sweep is the faster one, against the
+// tuned phase kernels.  A sweep of those on a lattice of this size costs its
+// launches, and how many there are depends on which directions pair up
+// (u1_duo.cuh).  One Metropolis and four overrelaxation passes, us, cluster /
+// phases (B200):
+//   2D: 128 x 256 (1024 sites) 20.5 / 26.7.
+//   3D: 24 x 28 x 34 (714) 36.9 / 38.9, 28^2 x 30 (735) 41.0 / 41.0, 30 x 26 x 34
+//       (829) 43.0 / 41.0, 32^3 (1024) 45.0 / 41.3.
+//   4D, two pairs (20 launches): 8^4 (128) 28.8 / 33.3, 8^3 x 12 (192) 34.8 / 36.9,
+//       8^2 x 10^2 (200) 36.9 / 34.8, 10^4 (315) 49.2 / 34.9 to 38.9, 12^4 (648)
+//       73.8 / 36.9 to 41.6 (as the tuner picked).  One block (6^3 x 4, 432): 26.7 / 34.8.
+//   4D, one pair (30): 10 x 12 x 10 x 12 (450) 59.4 / 60.4, 12 x 8 x 14 x 12 (504)
+//       59.4 / 61.4, 10^2 x 12 x 14 (525) 68.3 / 59.5.
+//   4D, none (40): 64 x 34 x 2 x 4 (544) 80.6 / 82.2.
+// Against the untuned default kernel the cluster wins wherever a block holds the
+// sites (4D, where it reads 19 links a site from other blocks' shared memory, up
+// to about 700: 12^4 73.8 / 86).
+static int cluster_most(const GeomK &g, bool tuned) {
+  if (g.dims == 2 || !tuned) return g.dims == 4 ? 704 : kClusterThreads;
+  if (g.dims == 3) return 768;
+  DuoK d;
+  return !duo_layout(g, 0, 256, d) ? 704 : duo_layout(g, 2, 256, d) ? 192 : 512;
+}
+
 // Whether the sweeps of `lat` run as one cluster launch (u1_cluster.cuh): a
 // lattice that fits, with an automatically chosen variant.  One block up to
 // 512 sites of a parity (its barrier costs about 0.3 us a phase, a
 // cluster's 0.6: 2D 32^2 10.4 us a sweep against 12.4), else 16 blocks
-// (8^4: 30.8 us; 8 blocks 33.1, 4 blocks 39.1; the phase kernels 71.8).  In
-// four dimensions distributed shared memory carries 19 link reads per site
-// and the gain is gone at about 700 sites per block (12^4, 648: 73.9 us
-// against 86.2), so larger 4D lattices keep the phase kernels; 2D and 3D
-// lattices use all 1024 threads (3D 32^3: 45.0 against 51.3).
+// (8^4: 30.8 us; 8 blocks 33.1, 4 blocks 39.1).
+// tunes: the caller tunes the phase kernels where the answer is no.
 // U1_CLUSTER=0 in the environment turns it off; the checked build takes it only
 // with U1_CLUSTER=1 (shared-memory addresses are checked, phases are not counted).
-static bool cluster_usable(u1_lattice *lat, int src) {
+static bool cluster_usable(u1_lattice *lat, int src, bool tunes = false) {
   if (lat->explicit_variant || src == SRC_REPLAY) return false;
   if (lat->cluster_ok < 0) {
     lat->cluster_ok = 0;
@@ -948,7 +969,8 @@ static bool cluster_usable(u1_lattice *lat, int src) {
 #endif
     if (env && env[0] == '0') return false;
     if (!cluster_layout(g, g.Vh <= 512 ? 1 : kClusterBlocks, lat->cluster)) return false;
-    if (g.dims == 4 && lat->cluster.threads > 704) return false;
+    if (lat->cluster.threads > cluster_most(g, false)) return false;
+    lat->cluster_most = lat->cluster.blocks == 1 ? kClusterThreads : cluster_most(g, true);
     const bool one = lat->cluster.blocks == 1;
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = cluster_config(lat, attr);
@@ -967,7 +989,8 @@ static bool cluster_usable(u1_lattice *lat, int src) {
     }
     lat->cluster_ok = 1;
   }
-  return lat->cluster_ok == 1;
+  return lat->cluster_ok == 1 &&
+         ((lat->variant == U1V_AUTO && !tunes) || lat->cluster.threads <= lat->cluster_most);
 }
 
 // Phase (1, MU) of the last pass with the measurement terms (u1_fused.cuh),
@@ -1490,8 +1513,9 @@ static int update_impl(u1_lattice *lat, u1_rng *rng, int metrop, int ovrn, doubl
   int rc = check_replay(lat, rng, metrop);
   if (rc) return rc;
   const bool replay = rng->replay_dev != nullptr;
-  const bool cluster = cluster_usable(lat, metropolis_src(lat, rng));  // worked out before a capture
-  if (lat->variant == U1V_AUTO && !replay && tuning_enabled()) {
+  const bool tunes = lat->variant == U1V_AUTO && !replay && tuning_enabled();
+  const bool cluster = cluster_usable(lat, metropolis_src(lat, rng), tunes);  // worked out before a capture
+  if (tunes) {
     if (cluster) {  // nothing to tune; the default kernel takes what stays phase by phase
       lat->variant = default_variant(lat->g);
     } else {
@@ -1544,7 +1568,7 @@ extern "C" int u1_update_measure(u1_lattice *lat, u1_rng *rng, int metrop, int o
   }
   int rc = u1i::ensure_scratch(lat, meas_sweep_scratch(lat->g), 8);
   if (rc) return rc;
-  if (cluster_usable(lat, metropolis_src(lat, rng))) {  // the sweep in one launch, then the measurement
+  if (cluster_usable(lat, metropolis_src(lat, rng), tuning_enabled())) {  // the sweep in one launch, then the measurement
     rc = update_impl(lat, rng, metrop, ovrn, nullptr);
     return rc ? rc : measure_dispatch(lat, dev_out);
   }

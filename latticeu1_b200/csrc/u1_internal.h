@@ -101,7 +101,8 @@ struct u1_lattice {
   int block = 256;                 // threads per block of the phase kernels (tuned with the variant)
   bool explicit_variant = false;   // a variant or block size was set (else chosen automatically)
   bool duo = false;                // two phases per launch, chosen by the tuner with U1V_SINGLE (u1_duo.cuh) or U1V_QUAD (u1_quad_duo.cu)
-  int cluster_ok = -1;             // sweeps as one cluster launch: -1 unknown, 0 no, 1 yes (layout: cluster)
+  int cluster_ok = -1;             // sweeps as one cluster launch: -1 unknown, 0 no, 1 possible (layout: cluster)
+  int cluster_most = 0;            // threads of its blocks up to which it beats the tuned phase kernels
   u1b::ClusterK cluster{};
   int remap_block = -1;            // block size remap_sms was worked out for
   int remap_sms = 0;               // SM-local block order of the four-site kernels (0: launch order)

@@ -12,6 +12,7 @@ import subprocess
 import sys
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 ROOT = Path(__file__).resolve().parents[1]
@@ -96,10 +97,17 @@ def test_block_size_selects_the_phase_kernels(ctx, monkeypatch):
     lat.close()
 
 
-@pytest.mark.parametrize("dims,N,tuned", [(4, (8, 8, 8, 8), False), (2, (32, 0, 0, 32), False),
-                                          (4, (16, 16, 16, 16), True)])
+# both sides of the lines between the cluster and the tuned phase kernels: one block,
+# 3D at 768 sites a block, 4D at 192 (two pairs of directions), 512 (one) and 704 (none)
+@pytest.mark.parametrize("dims,N,tuned", [
+    (4, (8, 8, 8, 8), False), (2, (32, 0, 0, 32), False), (2, (128, 0, 0, 256), False), (4, (6, 6, 6, 4), False),
+    (3, (28, 28, 0, 30), False), (3, (26, 30, 0, 32), True), (3, (32, 32, 0, 32), True),
+    (4, (8, 8, 8, 12), False), (4, (8, 8, 10, 10), True), (4, (12, 12, 12, 12), True),
+    (4, (12, 8, 14, 12), False), (4, (10, 10, 12, 14), True), (4, (64, 36, 2, 2), False),
+    (4, (16, 16, 16, 16), True)])
 def test_only_phase_kernels_are_tuned(ctx, dims, N, tuned, monkeypatch, tmp_path):
-    """The first update of a lattice on the cluster route times nothing: no trial, no line in the cache."""
+    """The cluster route up to where the tuned phase kernels overtake it; there the first update times
+    nothing: no trial, no line in the cache."""
     from latticeu1_b200 import Lattice, Rng
     monkeypatch.setenv("U1_RESOURCE_PATH", str(tmp_path))
     monkeypatch.delenv("U1_TUNE", raising=False)
@@ -114,7 +122,34 @@ def test_only_phase_kernels_are_tuned(ctx, dims, N, tuned, monkeypatch, tmp_path
     else:
         assert n == 1 and not lines
     assert lat.variant in (1, 2, 3, 5)
+    ref, rng_ref = Lattice(ctx, dims, N, 1.1), Rng(ctx, 5)
+    ref.set_variant(3)
+    ref.hot_start(rng_ref)
+    _launches(ref, rng_ref)
+    assert np.array_equal(lat.export_angles(), ref.export_angles())
     lat.close()
+    ref.close()
+
+
+def test_multilevel_of_an_untuned_lattice(ctx, monkeypatch):
+    """Sub-updates before and after a lattice beyond the line is tuned: another route, the same numbers."""
+    from latticeu1_b200 import Lattice, Rng
+    monkeypatch.delenv("U1_TUNE", raising=False)
+    monkeypatch.delenv("U1_CLUSTER", raising=False)
+    out = []
+    for variant, update in ((0, False), (0, True), (3, False)):
+        lat, rng = Lattice(ctx, 4, (8, 8, 10, 12), 0.95), Rng(ctx, 3)
+        if variant:
+            lat.set_variant(variant)
+        lat.hot_start(rng)
+        first = lat.multilevel(rng, 1, 1, 2, 1, 1, 1)
+        if update:
+            lat.tune(rng)
+        out.append((first, lat.multilevel(rng, 1, 1, 2, 1, 1, 1), lat.export_angles(), rng.state))
+        lat.close()
+    for o in out[1:]:
+        assert np.array_equal(o[0], out[0][0]) and np.array_equal(o[1], out[0][1])
+        assert np.array_equal(o[2], out[0][2]) and o[3] == out[0][3]
 
 
 def _child(route):

@@ -388,8 +388,9 @@ def e2e_rate(ctx, lat, rng, stream, N, beta, aniso, args, rank, world):
     for c in range(1, E2E_CHAINS):
         lc = Lattice(ctx, DIMS, N, beta, aniso)
         lc.set_metropolis(args.delta, args.nhits)
-        lc.set_variant(lat.variant)
-        lc.set_block(lat.block)
+        if args.variant:  # otherwise automatic as the first chain: the choice cached for the geometry,
+            lc.set_variant(args.variant)  # two phases per launch included
+            lc.set_block(args.block)
         sc = torch.cuda.Stream()
         lc.set_stream(sc.cuda_stream)
         rc_ = Rng(ctx, 1234)

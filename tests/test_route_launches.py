@@ -152,6 +152,52 @@ def test_multilevel_of_an_untuned_lattice(ctx, monkeypatch):
         assert np.array_equal(o[2], out[0][2]) and o[3] == out[0][3]
 
 
+def test_tuned_lattice_continues_its_chain(ctx, monkeypatch, tmp_path):
+    """A lattice beyond the cluster route after tune(): the tuned kernels run, and give the untuned one's links."""
+    from latticeu1_b200 import Lattice, Rng
+    monkeypatch.setenv("U1_RESOURCE_PATH", str(tmp_path))
+    monkeypatch.delenv("U1_CLUSTER", raising=False)
+    a, b = (Lattice(ctx, 4, (16, 16, 16, 8), 1.0) for _ in range(2))
+    ra, rb = Rng(ctx, 5), Rng(ctx, 5)
+    for lat, rng in ((a, ra), (b, rb)):
+        lat.set_variant(3)
+        lat.hot_start(rng)
+        lat.update(rng, 1, 2)
+    a.tune(ra)
+    assert 12 <= _launches(a, ra) <= 24 and _launches(b, rb) == 24
+    assert np.array_equal(a.export_angles(), b.export_angles()) and ra.state == rb.state
+    # another lattice of the geometry, left automatic, takes the choice over
+    c, rc = Lattice(ctx, 4, (16, 16, 16, 8), 1.0), Rng(ctx, 6)
+    c.hot_start(rc)
+    assert _launches(c, rc) == _launches(a, ra) and (c.variant, c.block) == (a.variant, a.block)
+
+
+def test_bench_chains_share_the_tuned_route(ctx, monkeypatch):
+    """The end-to-end chains beside the first one are left to the automatic choice: a variant and a block
+    size set from the first would run one phase per launch where it runs two."""
+    from types import SimpleNamespace
+
+    import torch
+
+    import bench
+    from latticeu1_b200 import Lattice, Rng
+    N = (16, 16, 16, 16)
+    lat, rng, stream = Lattice(ctx, 4, N, 1.0), Rng(ctx, 5), torch.cuda.Stream()
+    lat.set_stream(stream.cuda_stream)
+    lat.hot_start(rng)
+    lat.update(rng, 1, 4)
+    lat.synchronize()
+
+    def refuse(*a):
+        raise AssertionError("an automatic chain was given an explicit kernel")
+
+    monkeypatch.setattr(Lattice, "set_variant", refuse)
+    monkeypatch.setattr(Lattice, "set_block", refuse)
+    args = SimpleNamespace(delta=0.0, nhits=1, variant=0, block=0, steps=2)
+    rate, steps, finite = bench.e2e_rate(ctx, lat, rng, stream, N, 1.0, 1.0, args, 0, 1)
+    assert rate > 0 and steps == 6 and finite
+
+
 def _child(route):
     from latticeu1_b200 import Context, Lattice, Rng
     ctx = Context(0)

@@ -444,10 +444,11 @@ extern "C" int u1_batch_create(u1_ctx *ctx, int nchains, const u1_geom *geoms, u
     u1_batch_destroy(b);
     return rc;
   }
-  // cold start
+  // cold start (filled once on the host, for the largest chain)
+  std::vector<float2> one;
   for (int c = 0; c < nchains; ++c) {
     const size_t nl = (size_t)b->h_chains[c].g.V * b->h_chains[c].g.dims;
-    std::vector<float2> one(nl, make_float2(1.f, 0.f));
+    if (nl > one.size()) one.assign(nl, make_float2(1.f, 0.f));
     e = cudaMemcpy(b->h_chains[c].links, one.data(), nl * sizeof(float2), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
       u1_batch_destroy(b);

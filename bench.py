@@ -181,10 +181,12 @@ def update_kernel_digest() -> str:
     return h.hexdigest()[:16]
 
 
-def ncu_traffic_per_launch(N, kernel: str, profiles: Path | None = None) -> tuple[float | None, str]:
+def ncu_traffic_per_launch(N, kernel: str, profiles: Path | None = None,
+                           block: int | None = None) -> tuple[float | None, str]:
     """DRAM bytes per launch of `kernel` from the committed ncu summary for
     this geometry, and a note; None when there is no summary for this
-    geometry and kernel or it was made from other kernel sources."""
+    geometry and kernel, or it was made from other kernel sources or at
+    another block size than `block`."""
     p = (profiles or ROOT / "profiles") / f"k_update_{geom_name(N).replace('^4', 'x4')}_traffic.txt"
     if not p.exists():
         return None, f"no committed ncu summary for {geom_name(N)}"
@@ -194,6 +196,8 @@ def ncu_traffic_per_launch(N, kernel: str, profiles: Path | None = None) -> tupl
         return None, f"the committed ncu summary is for {fields.get('kernel')}, not {kernel}"
     if fields.get("source_digest") != update_kernel_digest():
         return None, "the committed ncu summary was made from other update-kernel sources (stale)"
+    if block is not None and fields.get("block", str(block)).split()[0] != str(block):
+        return None, f"the committed ncu summary was made at {fields['block']} threads per block, this run at {block}"
     return float(fields["dram_bytes_per_launch"].split()[0]), f"ncu, profiles/{p.name}"
 
 
@@ -532,7 +536,8 @@ def run_ours(args) -> None:
         avg_launch_s = upd_ms * 1e-3 / (args.steps * upd_launches)
         alg_bytes = algorithmic_bytes_per_link_update(DIMS) * volume(N) // 2
         achieved = alg_bytes / avg_launch_s / 1e9
-        traffic, traffic_note = ncu_traffic_per_launch(N, KERNEL_OF_VARIANT.get(lat.variant, "k_update"))
+        traffic, traffic_note = ncu_traffic_per_launch(N, KERNEL_OF_VARIANT.get(lat.variant, "k_update"),
+                                                       block=lat.block)
         l2_bytes = torch.cuda.get_device_properties(local).L2_cache_size
         resident = bytes_cfg < l2_bytes  # float2 links: 8 B each, as the FP64 angles
         line = {
@@ -819,7 +824,7 @@ def run_kernels(args) -> None:
     for _ in range(20):
         lat.update(rng, 1, 4)
     timed("u1_measure (plaquette + Polyakov)", "k_measure", lambda: lat.measure(), 8 * nl,
-          "reads every link once; 48 B result copy")
+          "reads every link once; 48 B stored to host memory")
     timed("u1_poly_corr(multihit=0)", "k_poly_field<4,0>, k_poly_corr", lambda: lat.poly_corr(False),
           8 * V + 16 * Vs, "temporal links, then the P field")
     timed("u1_poly_corr(multihit=1)", "k_poly_field<4,1>, k_poly_corr", lambda: lat.poly_corr(True),

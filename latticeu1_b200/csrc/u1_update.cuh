@@ -17,8 +17,6 @@
 
 namespace u1b {
 
-__device__ __forceinline__ float2 ldg2(const float2 *p) { return __ldg(p); }
-
 // Programmatic dependent launch (sm_90+): phase kernels are launched with
 // programmatic stream serialization, so the next phase's CTAs are scheduled
 // while this phase drains.  Every such kernel waits for the previous grid
@@ -548,10 +546,10 @@ __device__ __forceinline__ void update_pair_body(const UpdArgs a, int i, float2 
 // launch boundary and L2 round trips.  Row4 and 32-bit offsets within a half
 // lattice took the overrelaxation phase from 5.39 to 5.07 us at 32^4 and from
 // 3.67 to 3.28 us at 24^3 x 32; with 80 registers 3.15 us there, 28.6 -> 27.8
-// at 48^4 and 97 -> 94 at 64^4.  Two phases per launch (the chains that
-// directions 0, 1 or 2, 3 couple kept in a block), tiles of 2 x 4 x 4 rows per
-// block and a walk of the half-pass in L2-sized slabs were tried and are not
-// faster: 5.1, 6.0 and 6.2 us per 32^4 of sites.
+// at 48^4 and 97 -> 94 at 64^4.  Directions 0 and 1 of a half-pass also run as
+// one launch (u1_quad_duo.cu: 5.27 -> 4.95 us a phase at 32^4); directions 2 and 3
+// paired as well (5.1), tiles of 2 x 4 x 4 rows per block (6.0) and a walk of the
+// half-pass in L2-sized slabs (6.2 us per 32^4 of sites) are not faster.
 struct Quad2 {
   float2 s[4];
 };
